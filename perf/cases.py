@@ -235,15 +235,25 @@ def _bridge_arrays(case, seed):
             host(b), host(b2))
 
 
+def _on_grid(x, step, top):
+    """x rounded to multiples of `step`, at most `top` in size."""
+    return (x / step).round().mul_(step).clamp_(-top, top)
+
+
 def _layer_inputs(case, seed):
     """Activations after a ReLU (half of them zero), He-scaled weights, a
-    smooth-sized output gradient."""
+    small output gradient.  Activations and weights lie on binary grids (1/16
+    and 1/1024) on which a layer's sums are exact in 32 bits in any order:
+    whether a cell passes the ReLU, and with it every gradient, then never
+    hangs on the rounding of a value next to zero."""
     n = case["nx"] * case["ny"] * case["nz"]
     cin, cout = case["cin"], case["cout"]
     gen = torch.Generator(device="cuda").manual_seed(seed)
-    x = torch.randn(cin // 8, n, 8, generator=gen, device="cuda").relu().to(torch.bfloat16)
+    x = torch.randn(cin // 8, n, 8, generator=gen, device="cuda").relu()
+    x = _on_grid(x, 1.0 / 16, 4.0).to(torch.bfloat16)
     w = torch.randn(27, cout, cin, generator=gen, device="cuda") * math.sqrt(2.0 / (27 * cin))
-    b = torch.randn(cout, generator=gen, device="cuda") * 0.1
+    w = _on_grid(w, 1.0 / 1024, 0.25)
+    b = _on_grid(torch.randn(cout, generator=gen, device="cuda") * 0.1, 1.0 / 1024, 0.5)
     g = (torch.randn(cout // 8, n, 8, generator=gen, device="cuda") * 1e-2).to(torch.bfloat16)
     return x, w, b, g
 
