@@ -18,11 +18,12 @@
 // memory and the epilogue reads it with tcgen05.ld, adds the bias, applies
 // ReLU and stores BF16.
 //
-// Weight gradient: D[m = co][n = ci] = sum_cell dY[cell][co] X[cell+off][ci]
-// per tap, the cells being the K dimension: a CTA takes one tap and a range
-// of cells, stages dY^T (Cout rows, zero-padded to M = 128) and the shifted
-// X^T (Cin rows) K-major in shared memory, accumulates in TMEM, and adds its
-// partial [Cout][Cin] block into the FP32 gradient with atomics.
+// Weight gradient: the cells are the K dimension, and in the channel-blocked
+// layout 8 consecutive cells x 8 channels of a slab already form a core
+// matrix of a channel-major (MN-major) operand, so nothing is transposed: one
+// operand holds three copies shifted by the x taps, the other the y taps'
+// rows of three z planes, and every MMA forms a block of all 27 taps (the
+// layout and the roles are described at k_wgrad).
 //
 // Every mbarrier wait is bounded: on a timeout the kernel flags err, waits
 // (bounded again) for its MMAs in flight, frees its TMEM and returns.
@@ -60,28 +61,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n)
 {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
            ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem, uint64_t da, uint64_t db,
-                                          uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t *mbar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(smem_u32(mbar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *m)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(m)));
 }
 
 __device__ __forceinline__ bool mbar_test(uint64_t *m, unsigned parity)
@@ -168,11 +147,6 @@ __device__ __forceinline__ void tmem_ld16_nw(uint32_t taddr, float v[16])
 __device__ __forceinline__ void tmem_wait_ld()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__host__ __device__ constexpr int tmem_cols(int n)
-{
-    return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256;
 }
 
 // ---- forward / data gradient ----------------------------------------------
@@ -675,150 +649,261 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
 }
 
 // ---- weight gradient --------------------------------------------------------
-
-constexpr int kWgCells = 64;  // cells (K) staged per round: 4 MMAs of K = 16
-
-template <int CIN, int COUT>
-struct WgSmem {
-    // A: dY^T, 128 rows (COUT used, rest zero) x kWgCells; B: X^T, CIN rows
-    static constexpr int kA = 128 * kWgCells * 2;
-    static constexpr int kB = CIN * kWgCells * 2;
-    static constexpr int kBytes = 2 * kA + 2 * kB + 64;
+//
+// dW[tap][co][ci] = sum_c dY[c][co] X[c + tap][ci].  Writing the tap as a sum
+// of an x shift on one side and a (y, z) shift on the other,
+//     D[(dx, m)][(z plane, y row, n)] = sum_p M[p + dx][m] N[p + (y, z)][n],
+// with M and N the two tensors in the order that wastes less (WgPlan::flip:
+// M = dY, N = X), one MMA has all three x taps in its rows and the y and z
+// taps in its columns: with 16 -> 16 channels 48 x 144 useful entries of
+// 128 x 144 for 16 cells, against 16 x 16 of 128 x 16 for one tap per MMA
+// (one tap per CTA, both operands transposed through registers).  Measured
+// against that form: 16 -> 16 at 128^3 2707 -> 136 us, 48 -> 16 3814 -> 262,
+// 96 -> 32 at 64^3 1335 -> 106, 64 -> 64 at 32^3 125 -> 32.  What bounds it
+// now are the group copies (16 -> 16: 12 groups for each 128 x 144 MMA).
+//
+// A step is 32 x BY cells of one z plane.  A group is one slab (8 channels)
+// of a step, BY rows of 32 cells, 16 bytes a cell: an MN-major operand
+// without swizzle whose K groups (8 cells) lie 128 bytes and whose 8-channel
+// groups SP = 512 BY bytes apart.  Tensor copies bring the groups in and
+// fill what lies outside the grid (x, y or z) with zeros, so no tile edge
+// has a case of its own: the M side as 3 x slabs groups at x - 1, x, x + 1,
+// the N side per z plane as 3 x NS groups at y - 1, y, y + 1.  A CTA walks
+// z, so each N plane is loaded once for its three z taps (a ring of RN
+// planes); M planes go through a ring of RM stages.  Groups of the A operand
+// beyond the tensor's (M = 128 is 16 groups) read whatever shared memory
+// follows: their rows of D are never looked at.
+//
+// A part is one block of 16 M groups and NS slabs of N; a CTA keeps one
+// part's D in tensor memory over all its cells and adds it into dw at the
+// end.  Roles: warp 4 loads (a lane per group), warp 5 issues, warps 0-3
+// read D.
+struct WgPlan {
+    int flip;              // 0: M = x, N = dy; 1: M = dy, N = x
+    int ms, gm, gmax;      // M side: slabs, groups (3 ms), groups per stage
+    int mblk, parts;       // M blocks; parts = mblk x (N slabs / NS)
+    int cin, cout;
+    int nxc, nyb, zl, nzc; // 32-cell columns, BY-row blocks, z planes per item, items along z
+    int per;               // CTAs per part
+    int vec;               // dw is 16-byte aligned
 };
 
-// grid (cell blocks, 27 taps); each CTA: tap blockIdx.y, cells
-// [blockIdx.x * per_cta, +per_cta)
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128)
-k_conv3d_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy,
-               float *__restrict__ dw, int nx, int ny, int nz, long per_cta, int *err)
-{
-    static_assert(CIN % 16 == 0 && CIN <= 256 && COUT <= 128 && COUT % 8 == 0, "channels");
-    extern __shared__ __align__(128) unsigned char smem[];
-    using S = WgSmem<CIN, COUT>;
-    unsigned char *abuf = smem, *bbuf = smem + 2 * S::kA;
-    uint64_t *mbar = (uint64_t *)(smem + 2 * S::kA + 2 * S::kB);
-    uint32_t *tslot = (uint32_t *)(mbar + 2);
-    constexpr int NCOL = tmem_cols(CIN);
-    constexpr uint32_t IDESC = idesc_bf16(128, CIN);
-    constexpr int KCH = kWgCells / 8;  // 16-byte K chunks per round
+template <int NS, int BY>
+struct WgCfg {
+    static constexpr int SP = BY * 512;        // bytes of a group
+    static constexpr int KS = BY * 2;          // MMAs (16 cells) along K per step
+    static constexpr int GN = 3 * NS;          // groups of an N plane
+    static constexpr int COLS = 72 * NS;       // columns of D: 3 planes x GN x 8
+    static constexpr int TCOLS = COLS <= 256 ? 256 : 512;
+    static constexpr int RM = BY == 4 ? 3 : 4;
+    static constexpr int RN = BY == 4 ? 6 : NS == 4 ? 8 : 7;
+    static constexpr int kBytes(int gmax) { return (RM * gmax + RN * GN) * SP + 256; }
+};
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int tap = blockIdx.y;
-    const int dx = tap % 3 - 1, dyy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-    const long nxy = (long)nx * ny, n = nxy * nz;
-    const long c_begin = (long)blockIdx.x * per_cta;
-    const long c_end = c_begin + per_cta < n ? c_begin + per_cta : n;
+// kind::f16 with both operands MN-major (bits 15 and 16)
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n)
+{
+    return idesc_bf16(m, n) | (1u << 15) | (1u << 16);
+}
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1,
+                                            int c2, int c3, uint64_t *m)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(m))
+        : "memory");
+}
+
+template <int NS, int BY>
+__global__ void __launch_bounds__(kConvThreads, 1)
+k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_n,
+        float *__restrict__ dw, int nz, const WgPlan p, int *err)
+{
+    using C = WgCfg<NS, BY>;
+    constexpr int SP = C::SP, GN = C::GN, RM = C::RM, RN = C::RN;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int mstage = p.gmax * SP;
+    unsigned char *mring = smem, *nring = smem + RM * mstage;
+    uint64_t *bar = (uint64_t *)(nring + RN * GN * SP);
+    uint64_t *full_m = bar, *empty_m = bar + RM, *full_n = bar + 2 * RM, *empty_n = full_n + RN,
+             *done = empty_n + RN;
+    uint32_t *tslot = (uint32_t *)(done + 1);
+    volatile int *abort_flag = (volatile int *)(tslot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int part = blockIdx.x % p.parts, idx = blockIdx.x / p.parts;
+    const int g0 = 16 * (part % p.mblk), s0 = NS * (part / p.mblk);
+    const int gmc = p.gm - g0 < 16 ? p.gm - g0 : 16;
+    const long items = (long)p.nxc * p.nyb * p.nzc;
     if (tid == 0) {
-        mbar_init(&mbar[0]);
-        mbar_init(&mbar[1]);
+        for (int i = 0; i < 2 * RM + 2 * RN + 1; i++) mbar_init_n(&bar[i], 1);
+        *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // rows COUT..127 of both A buffers stay zero
-    for (int i = tid; i < 2 * S::kA / 16; i += 128) ((uint4 *)abuf)[i] = make_uint4(0, 0, 0, 0);
-    if (warp == 0) tmem_alloc(tslot, NCOL);
+    if (warp == 5) tmem_alloc(tslot, C::TCOLS);
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
     const uint32_t tmem = *tslot;
-    unsigned parity[2] = {0u, 0u};
-    int pending[2] = {0, 0};
-    bool ok = true, any = false;
-    int round = 0;
-    for (long c0 = c_begin; c0 < c_end && ok; c0 += kWgCells, round++) {
-        const int b = round & 1;
-        if (pending[b]) {
-            ok = mbar_wait(&mbar[b], parity[b]);
-            parity[b] ^= 1u;
-            pending[b] = 0;
-            ok = __syncthreads_and(ok);
-            if (!ok) break;
+
+    if (warp == 4) {
+        long mseq = 0, nseq = 0;
+        // this lane's group: of the M side (x shift, slab), of an N plane
+        // (y shift, slab)
+        const int gi = (g0 + lane) / p.ms, gs = (g0 + lane) % p.ms;
+        const int nj = lane / NS, nslab = s0 + lane % NS;
+        bool ok = true;
+        for (long it = idx; it < items && ok; it += p.per) {
+            const int xc = (int)(it % p.nxc), yb = (int)((it / p.nxc) % p.nyb),
+                      zc = (int)(it / ((long)p.nxc * p.nyb));
+            const int z0 = zc * p.zl, z1 = z0 + p.zl < nz ? z0 + p.zl : nz;
+            for (int z = z0 - 1; z <= z1; z++) {  // N plane z, then M plane z - 1
+                const int sn = (int)(nseq % RN);
+                if (!__all_sync(0xffffffffu,
+                                role_wait(&empty_n[sn], ((unsigned)(nseq / RN) & 1u) ^ 1u,
+                                          abort_flag, err))) {
+                    ok = false;
+                    break;
+                }
+                if (lane == 0) mbar_expect_tx_only(&full_n[sn], GN * SP);
+                __syncwarp();
+                if (lane < GN)
+                    tma_load_4d(smem_u32(nring + (sn * GN + lane) * SP), &tm_n, 256 * xc,
+                                BY * yb + nj - 1, z, nslab, &full_n[sn]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full_n[sn]);
+                nseq++;
+                if (z <= z0) continue;
+                const int sm = (int)(mseq % RM);
+                if (!__all_sync(0xffffffffu,
+                                role_wait(&empty_m[sm], ((unsigned)(mseq / RM) & 1u) ^ 1u,
+                                          abort_flag, err))) {
+                    ok = false;
+                    break;
+                }
+                if (lane == 0) mbar_expect_tx_only(&full_m[sm], (uint32_t)(gmc * SP));
+                __syncwarp();
+                if (lane < gmc)
+                    tma_load_4d(smem_u32(mring + sm * mstage + lane * SP), &tm_m,
+                                256 * xc + 8 * (gi - 1), BY * yb, z - 1, gs, &full_m[sm]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full_m[sm]);
+                mseq++;
+            }
         }
-        unsigned char *a = abuf + b * S::kA, *bb = bbuf + b * S::kB;
-        // A[co][k] = dY[c0 + k][co]: thread k-pair stages the COUT values of
-        // two cells (element (row co, k) at (k/8)*2048 + co*16 + (k%8)*2)
-        for (int k = tid; k < kWgCells; k += 128) {
-            const long cell = c0 + k;
-            const bool v = cell < c_end;
-            for (int co = 0; co < COUT; co += 8) {
-                uint4 q = v ? *(const uint4 *)(dy + ((long)(co / 8) * n + cell) * 8)
-                            : make_uint4(0, 0, 0, 0);
-                const __nv_bfloat16 *e = (const __nv_bfloat16 *)&q;
+        // copies still in flight land before the CTA leaves
+        if (lane == 0) {
+            for (int j = 0; j < RN && j < nseq; j++) {
+                const long q = nseq - 1 - j;
+                if (!mbar_wait(&full_n[q % RN], (unsigned)(q / RN) & 1u)) atomicExch(err, 1);
+            }
+            for (int j = 0; j < RM && j < mseq; j++) {
+                const long q = mseq - 1 - j;
+                if (!mbar_wait(&full_m[q % RM], (unsigned)(q / RM) & 1u)) atomicExch(err, 1);
+            }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        long mseq = 0, nseq = 0;
+        bool ok = true;
+        uint32_t acc = 0;  // nothing in D yet
+        const uint32_t nbase = smem_u32(nring), mbase = smem_u32(mring);
+        for (long it = idx; it < items && ok; it += p.per) {
+            const int zc = (int)(it / ((long)p.nxc * p.nyb));
+            const int z0 = zc * p.zl, z1 = z0 + p.zl < nz ? z0 + p.zl : nz;
+            for (int z = z0; z < z1 && ok; z++, nseq++, mseq++) {
+                // planes z - 1, z, z + 1 are ring items nseq .. nseq + 2
+                for (int k = z == z0 ? 0 : 2; k < 3; k++)
+                    ok = ok && __all_sync(0xffffffffu,
+                                          role_wait(&full_n[(nseq + k) % RN],
+                                                    (unsigned)((nseq + k) / RN) & 1u, abort_flag,
+                                                    err));
+                const int sm = (int)(mseq % RM);
+                ok = ok && __all_sync(0xffffffffu, role_wait(&full_m[sm],
+                                                             (unsigned)(mseq / RM) & 1u,
+                                                             abort_flag, err));
+                if (!ok) break;
+                tc_after_sync();
+                const uint64_t da = kmajor_desc(mbase + (uint32_t)(sm * mstage), 128, SP);
+                const int r0 = (int)(nseq % RN);
+                uint64_t db[3];
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    *(__nv_bfloat16 *)(a + (k / 8) * 2048 + (co + j) * 16 + (k % 8) * 2) = e[j];
-            }
-        }
-        // B[ci][k] = X[cell + off][ci] (zero outside the grid)
-        for (int k = tid; k < kWgCells; k += 128) {
-            const long cell = c0 + k;
-            bool v = cell < c_end;
-            long src = 0;
-            if (v) {
-                const int xx = (int)(cell % nx) + dx, yy = (int)((cell / nx) % ny) + dyy,
-                          zz = (int)(cell / nxy) + dz;
-                v = xx >= 0 && xx < nx && yy >= 0 && yy < ny && zz >= 0 && zz < nz;
-                src = xx + (long)yy * nx + (long)zz * nxy;
-            }
-            for (int ci = 0; ci < CIN; ci += 8) {
-                uint4 q = v ? *(const uint4 *)(x + ((long)(ci / 8) * n + src) * 8)
-                            : make_uint4(0, 0, 0, 0);
-                const __nv_bfloat16 *e = (const __nv_bfloat16 *)&q;
+                for (int k = 0; k < 3; k++)
+                    db[k] = kmajor_desc(nbase + (uint32_t)(((nseq + k) % RN) * GN * SP), 128, SP);
+                // one MMA over the three planes where they are consecutive
+                // in the ring and N = 3 GN 8 <= 256, otherwise one per plane
+                const bool one = C::COLS <= 256 && r0 + 2 < RN;
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    *(__nv_bfloat16 *)(bb + (k / 8) * (CIN * 16) + (ci + j) * 16 + (k % 8) * 2) =
-                        e[j];
-            }
-        }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_after_sync();
-            const uint32_t sa = smem_u32(a), sb = smem_u32(bb);
+                for (int ks = 0; ks < C::KS; ks++) {
+                    const uint64_t o = (uint64_t)(16 * ks);  // 256 bytes
+                    if (one) {
+                        umma_bf16_elect(tmem, da + o, db[0] + o,
+                                        idesc_bf16_mn(128, C::COLS <= 256 ? C::COLS : 256), acc);
+                    } else {
 #pragma unroll
-            for (int kk = 0; kk < KCH / 2; kk++) {
-                const uint64_t da = kmajor_desc(sa + kk * 2 * 2048, 2048, 128);
-                const uint64_t db = kmajor_desc(sb + kk * 2 * (CIN * 16), CIN * 16, 128);
-                umma_bf16(tmem, da, db, IDESC, (round | kk) != 0);
+                        for (int k = 0; k < 3; k++)
+                            umma_bf16_elect(tmem + (uint32_t)(k * GN * 8), da + o, db[k] + o,
+                                            idesc_bf16_mn(128, GN * 8), acc);
+                    }
+                    acc = 1;
+                }
+                umma_commit_elect(&empty_m[sm]);
+                umma_commit_elect(&empty_n[r0]);
+                if (z == z1 - 1) {  // the walk's last two planes
+                    umma_commit_elect(&empty_n[(nseq + 1) % RN]);
+                    umma_commit_elect(&empty_n[(nseq + 2) % RN]);
+                }
             }
-            umma_commit(&mbar[b]);
+            nseq += 2;
         }
-        pending[b] = 1;
-        any = true;
-    }
-    if (ok) {
-        for (int b = 0; b < 2; b++) {
-            if (pending[b]) {
-                ok = ok && mbar_wait(&mbar[b], parity[b]);
-                parity[b] ^= 1u;
-                pending[b] = 0;
-            }
+        umma_commit_elect(done);
+        if (lane == 0 && !mbar_wait(done, 0)) {
+            *abort_flag = 1;
+            atomicExch(err, 1);
         }
-        ok = __syncthreads_and(ok);
-    }
-    if (ok && any) {
+        __syncwarp();
+    } else if (__all_sync(0xffffffffu, role_wait(done, 0, abort_flag, err) && !*abort_flag)) {
         tc_after_sync();
-        // row co = 32 warp + lane of D, columns ci
-        const int co = 32 * warp + (tid & 31);
+        const int g = g0 + 4 * warp + (lane >> 3);  // row 32 warp + lane: group, channel
+        const bool v = g < p.gm;
+        const int i = v ? g / p.ms : 0, cm = v ? 8 * (g % p.ms) + (lane & 7) : 0;
 #pragma unroll 1
-        for (int c = 0; c < CIN; c += 16) {
-            float v[16];
-            tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, v);
-            if (co < COUT)
+        for (int c = 0; c < C::COLS; c += 16) {
+            float f[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, f);
+            if (!v) continue;
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    atomicAdd(&dw[((long)tap * COUT + co) * CIN + c + i], v[i]);
+            for (int h = 0; h < 2; h++) {
+                const int q = c / 8 + h, k = q / GN, j = (q / NS) % 3;
+                const int cn = 8 * (s0 + q % NS);
+                if (!p.flip) {
+                    // X at p + (i-1), dY at p + (j-1, k-1): tap (i-1, 1-j, 1-k)
+                    const int tap = 9 * (2 - k) + 3 * (2 - j) + i;
+                    float *o = dw + ((long)tap * p.cout + cn) * p.cin + cm;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) atomicAdd(o + (long)e * p.cin, f[8 * h + e]);
+                } else {
+                    // dY at p + (i-1), X at p + (j-1, k-1): tap (1-i, j-1, k-1)
+                    const int tap = 9 * k + 3 * j + (2 - i);
+                    float *o = dw + ((long)tap * p.cout + cm) * p.cin + cn;
+                    if (p.vec) {
+                        atomicAdd((float4 *)o, make_float4(f[8 * h], f[8 * h + 1], f[8 * h + 2],
+                                                           f[8 * h + 3]));
+                        atomicAdd((float4 *)o + 1, make_float4(f[8 * h + 4], f[8 * h + 5],
+                                                               f[8 * h + 6], f[8 * h + 7]));
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) atomicAdd(o + e, f[8 * h + e]);
+                    }
+                }
+            }
         }
-    }
-    if (!ok) {
-        if (tid == 0) atomicExch(err, 1);
-        for (int b = 0; b < 2; b++)
-            if (pending[b]) mbar_wait(&mbar[b], parity[b]);
     }
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
-    if (warp == 0) tmem_free(tmem, NCOL);
+    if (warp == 5) tmem_free(tmem, C::TCOLS);
 }
 
 // Tile choice for a forward launch: row mode (bx = 128) or plane mode (bx =
@@ -980,29 +1065,94 @@ int launch_fwd(const void *in, const void *w, const float *bias, void *out, int 
     return HMFEM_OK;
 }
 
-template <int CIN, int COUT>
-int launch_wgrad(const void *x, const void *dy, float *dw, int nx, int ny, int nz, int *err,
-                 cudaStream_t st)
+// N slabs per part: all of them where 9 x 8 NS columns fit in tensor memory
+constexpr int wgrad_ns(int cn) { return cn == 16 ? 2 : cn == 32 || cn == 64 ? 4 : 6; }
+
+// Estimated cycles per 16 cells of every part with these M and N channels:
+// N / 2 per MMA (M = 128 rows are the array's full height), or the shared
+// memory's 128 bytes a cycle where operands and incoming groups need longer.
+double wgrad_cost(int cm, int cn)
 {
-    using S = WgSmem<CIN, COUT>;
-    auto k = k_conv3d_wgrad<CIN, COUT>;
-    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
-    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    const long n = (long)nx * ny * nz;
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    // ~4 waves of CTAs over the 27 taps, whole rounds of kWgCells cells each
-    long blocks_x = (4L * nsm + 26) / 27;
-    long per = (n + blocks_x - 1) / blocks_x;
-    per = (per + kWgCells - 1) / kWgCells * kWgCells;
-    if (per < kWgCells) per = kWgCells;
-    blocks_x = (n + per - 1) / per;
-    k<<<dim3((unsigned)blocks_x, 27), 128, S::kBytes, st>>>((const __nv_bfloat16 *)x,
-                                                           (const __nv_bfloat16 *)dy, dw, nx,
-                                                           ny, nz, per, err);
+    const int ns = wgrad_ns(cn), mblk = (3 * cm / 8 + 15) / 16, nblk = cn / 8 / ns;
+    const double mma = 36.0 * ns;
+    const int gmax = 3 * cm / 8 < 16 ? 3 * cm / 8 : 16;
+    const double smem = ((ns == 2 ? 1 : 3) * 4096.0 + 72.0 * ns * 32 + (gmax + 3 * ns) * 256.0) / 128;
+    return mblk * nblk * (mma > smem ? mma : smem);
+}
+
+template <int NS, int BY>
+int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, int nx, int ny,
+                     int nz, WgPlan p, int nsm, int *err, cudaStream_t st)
+{
+    using C = WgCfg<NS, BY>;
+    p.ms = cm / 8;
+    p.gm = 3 * p.ms;
+    p.gmax = p.gm < 16 ? p.gm : 16;
+    p.mblk = (p.gm + 15) / 16;
+    p.parts = p.mblk * (cn / 8 / NS);
+    p.nxc = (nx + 31) / 32;
+    p.nyb = (ny + BY - 1) / BY;
+    // CTAs per part: the SMs' share, but no fewer than ~16 steps each (every
+    // CTA adds its whole D into dw at the end)
+    const long cols = (long)p.nxc * p.nyb;
+    long per = nsm / p.parts < 1 ? 1 : nsm / p.parts;
+    const long by_work = (cols * nz + 15) / 16;
+    if (per > by_work) per = by_work;
+    // z planes per item: an item of zl planes loads zl + 2 N planes; the
+    // makespan is the items of the fullest CTA
+    double best = 1e300;
+    p.zl = nz;
+    for (int c = 1; c <= nz; c++) {
+        const int zl = (nz + c - 1) / c, zc = (nz + zl - 1) / zl;
+        const double t = (double)((cols * zc + per - 1) / per) * (zl + 1.5);
+        if (t < best) {
+            best = t;
+            p.zl = zl;
+        }
+    }
+    p.nzc = (nz + p.zl - 1) / p.zl;
+    if (per > cols * p.nzc) per = cols * p.nzc;
+    p.per = (int)per;
+    p.vec = ((uintptr_t)dw & 15u) == 0;
+    CUtensorMap tm[2];
+    const void *base[2] = {m, nn};
+    const int ch[2] = {cm, cn};
+    for (int i = 0; i < 2; i++) {
+        const cuuint64_t dims[4] = {(cuuint64_t)nx * 8, (cuuint64_t)ny, (cuuint64_t)nz,
+                                    (cuuint64_t)ch[i] / 8};
+        const cuuint64_t strides[3] = {(cuuint64_t)nx * 16, (cuuint64_t)nx * ny * 16,
+                                       (cuuint64_t)nx * ny * nz * 16};
+        const cuuint32_t box[4] = {256, (cuuint32_t)BY, 1, 1};
+        const int rc = encode_bf16_map(&tm[i], base[i], 4, dims, strides, box);
+        if (rc != HMFEM_OK) return rc;
+    }
+    const int bytes = C::kBytes(p.gmax);
+    // the A operand's 16 groups from the last M stage stay inside the buffer
+    static_assert(16 * C::SP <= C::RN * C::GN * C::SP, "operand overrun");
+    auto k = k_wgrad<NS, BY>;
+    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    k<<<(unsigned)(per * p.parts), kConvThreads, bytes, st>>>(tm[0], tm[1], dw, nz, p, err);
     HM_LAUNCHED();
     return HMFEM_OK;
+}
+
+int launch_wgrad(const void *x, const void *dy, float *dw, int nx, int ny, int nz, int cin,
+                 int cout, int *err, cudaStream_t st)
+{
+    int dev = 0, nsm = 0;
+    HM_CUDA(cudaGetDevice(&dev));
+    HM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    WgPlan p{};
+    p.cin = cin;
+    p.cout = cout;
+    p.flip = wgrad_cost(cout, cin) < wgrad_cost(cin, cout);
+    const void *m = p.flip ? dy : x, *nn = p.flip ? x : dy;
+    const int cm = p.flip ? cout : cin, cn = p.flip ? cin : cout;
+    switch (wgrad_ns(cn)) {
+    case 2: return launch_wgrad_cfg<2, 4>(m, nn, cm, cn, dw, nx, ny, nz, p, nsm, err, st);
+    case 4: return launch_wgrad_cfg<4, 2>(m, nn, cm, cn, dw, nx, ny, nz, p, nsm, err, st);
+    default: return launch_wgrad_cfg<6, 2>(m, nn, cm, cn, dw, nx, ny, nz, p, nsm, err, st);
+    }
 }
 
 #define HM_CONV_SHAPES(X)                                                                \
@@ -1049,7 +1199,7 @@ int hmfem_conv3d_wgrad(const void *x, const void *dy, float *dw, int nx, int ny,
     if (!x || !dy || !dw || !err || nx < 1 || ny < 1 || nz < 1) return HMFEM_E_ARG;
     cudaStream_t st = (cudaStream_t)stream;
 #define X(a, b)                                                                               \
-    if (cin == a && cout == b) return hm::launch_wgrad<a, b>(x, dy, dw, nx, ny, nz, err, st);
+    if (cin == a && cout == b) return hm::launch_wgrad(x, dy, dw, nx, ny, nz, a, b, err, st);
     HM_CONV_SHAPES(X)
 #undef X
     hm::set_last_error("conv3d: unsupported channel counts", __FILE__, __LINE__);

@@ -117,6 +117,57 @@ __global__ void k_up2_grad(const __nv_bfloat16 *__restrict__ g, int Sa, int nx, 
     ((uint4 *)out)[i] = *(uint4 *)o;
 }
 
+// The ReLU's gradient and the bias gradient in one pass: g = gout * (out > 0)
+// (out NULL: no ReLU, g not written) and, per slab, the block's sum of g over
+// its cells in FP32 (part[slab][block][8], added up in FP64 by k_bias_sum).
+// Bound by HBM, 6 bytes a value: 40 us at 128^3 x 16 channels, against
+// 286 us for the mask, the product, the conversion and the sum one by one.
+__global__ void __launch_bounds__(kOpsThreads)
+k_relu_grad(const __nv_bfloat16 *__restrict__ gout, const __nv_bfloat16 *__restrict__ out,
+            long n, __nv_bfloat16 *__restrict__ g, float *__restrict__ part)
+{
+    const long base = (long)blockIdx.y * n;
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (long s = (long)blockIdx.x * kOpsThreads + threadIdx.x; s < n;
+         s += (long)gridDim.x * kOpsThreads) {
+        uint4 q = ((const uint4 *)gout)[base + s];
+        __nv_bfloat16 *e = (__nv_bfloat16 *)&q;
+        if (out) {
+            const uint4 a = ((const uint4 *)out)[base + s];
+            const __nv_bfloat16 *o = (const __nv_bfloat16 *)&a;
+#pragma unroll
+            for (int j = 0; j < 8; j++)  // a product, as NaN and -0 behave in one
+                e[j] = __float2bfloat16(__bfloat162float(e[j]) *
+                                        (__bfloat162float(o[j]) > 0.f ? 1.f : 0.f));
+            ((uint4 *)g)[base + s] = q;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j] += __bfloat162float(e[j]);
+    }
+    __shared__ float sh[kOpsThreads / 32][8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        acc[j] = warp_sum(acc[j]);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][j] = acc[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        float t = 0.f;
+        for (int w = 0; w < kOpsThreads / 32; w++) t += sh[w][threadIdx.x];
+        part[((long)blockIdx.y * gridDim.x + blockIdx.x) * 8 + threadIdx.x] = t;
+    }
+}
+
+// gb[channel] from the blocks' sums: a warp per channel
+__global__ void k_bias_sum(const float *__restrict__ part, int blocks, float *__restrict__ gb)
+{
+    const int c = blockIdx.x, lane = threadIdx.x;
+    double t = 0.0;
+    for (int b = lane; b < blocks; b += 32) t += part[((long)(c / 8) * blocks + b) * 8 + c % 8];
+    t = warp_sum(t);
+    if (lane == 0) gb[c] = (float)t;
+}
+
 // p[s] = 1 - (x + 1/2)/nx + (sum_c x[c] w[c] + b): the 1x1 head (FP32) on the
 // linear profile, FP64 out
 __global__ void k_head_profile(const __nv_bfloat16 *__restrict__ x, int S,
@@ -192,6 +243,24 @@ int hmfem_guess_up2_grad(const void *g, int slabs_a, int nx, int ny, int nz, voi
     const long work = (long)slabs_a * (nx / 2) * (ny / 2) * (nz / 2);
     hm::k_up2_grad<<<hm::ops_grid(work), hm::kOpsThreads, 0, (cudaStream_t)stream>>>(
         (const __nv_bfloat16 *)g, slabs_a, nx, ny, nz, (__nv_bfloat16 *)out);
+    HM_LAUNCHED();
+    return HMFEM_OK;
+}
+
+int hmfem_guess_relu_grad(const void *gout, const void *out, int slabs, long n, void *g,
+                          float *gb, float *part, int blocks, void *stream)
+{
+    if (!gout || !gb || !part || slabs < 1 || slabs > 65535 || n < 1 || blocks < 1 || (out && !g))
+        return HMFEM_E_ARG;
+    if (((uintptr_t)gout | (uintptr_t)out | (uintptr_t)g) & 15u) {
+        hm::set_last_error("guess relu_grad: tensors must be 16-byte aligned", __FILE__, __LINE__);
+        return HMFEM_E_ARG;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    hm::k_relu_grad<<<dim3(blocks, slabs), hm::kOpsThreads, 0, st>>>(
+        (const __nv_bfloat16 *)gout, (const __nv_bfloat16 *)out, n, (__nv_bfloat16 *)g, part);
+    HM_LAUNCHED();
+    hm::k_bias_sum<<<8 * slabs, 32, 0, st>>>(part, blocks, gb);
     HM_LAUNCHED();
     return HMFEM_OK;
 }

@@ -45,6 +45,7 @@ def _lib():
         L.hmfem_guess_pool2.argtypes = [vp, i, i, i, i, vp, vp]
         L.hmfem_guess_up2_cat.argtypes = [vp, i, vp, i, i, i, i, vp, vp]
         L.hmfem_guess_up2_grad.argtypes = [vp, i, i, i, i, vp, vp]
+        L.hmfem_guess_relu_grad.argtypes = [vp, vp, i, C.c_long, vp, vp, vp, i, vp]
         L.hmfem_guess_head_profile.argtypes = [vp, i, vp, vp, i, i, i, vp, vp]
         L._guess_bound = True
     return L
@@ -131,6 +132,22 @@ def conv3d_wgrad_raw(x, dy, dims):
     return dw
 
 
+def relu_grad_raw(gout, out):
+    """(g, gb): g = gout * (out > 0) (out None: g is gout) and its sums over
+    the cells (FP32); gout, out (c/8, n, 8) bf16."""
+    gout = gout.contiguous()
+    slabs, n, _ = gout.shape
+    g = gout if out is None else torch.empty_like(gout)
+    gb = torch.empty(8 * slabs, dtype=torch.float32, device=gout.device)
+    # ~4 blocks an SM over all slabs, a block no less than four rounds of cells
+    blocks = max(1, min(600 // slabs, n // 1024))
+    part = torch.empty(8 * slabs * blocks, dtype=torch.float32, device=gout.device)
+    _rc(_lib().hmfem_guess_relu_grad(gout.data_ptr(), None if out is None else out.data_ptr(),
+                                     slabs, n, None if out is None else g.data_ptr(),
+                                     gb.data_ptr(), part.data_ptr(), blocks, _stream(gout)))
+    return g, gb
+
+
 def flip_transpose(w):
     """Weights of the data gradient: w_t[t][ci][co] = w[26 - t][co][ci]."""
     return w.flip(0).transpose(1, 2).contiguous()
@@ -148,12 +165,9 @@ class Conv3x3x3(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gout):
         x, wb, out = ctx.saved_tensors
-        g = gout.to(torch.bfloat16)
-        if ctx.relu:
-            g = g * (out > 0).to(g.dtype)
+        g, gb = relu_grad_raw(gout.to(torch.bfloat16), out if ctx.relu else None)
         gx = conv3d_raw(g, flip_transpose(wb), None, ctx.dims, False)
         gw = conv3d_wgrad_raw(x, g, ctx.dims)
-        gb = g.float().sum(1).reshape(-1)
         return gx, gw, gb, None, None
 
 

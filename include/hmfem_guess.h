@@ -43,6 +43,13 @@ int hmfem_conv3d_plan(int nx, int ny, int nz, int cin, int cout, int nsm, int sm
 int hmfem_conv3d_wgrad(const void *x, const void *dy, float *dw, int nx, int ny, int nz,
                        int cin, int cout, int *err, void *stream);
 
+/* The gradient through a layer's ReLU and its bias gradient (BF16 slabs of n
+ * cells): g = gout * (out > 0), gb[8 slabs] = the sums of g over the cells
+ * (FP32).  out NULL: no ReLU, g (NULL) is not written and gb sums gout.
+ * part: scratch of 8 * slabs * blocks floats; blocks: thread blocks per slab. */
+int hmfem_guess_relu_grad(const void *gout, const void *out, int slabs, long n, void *g,
+                          float *gb, float *part, int blocks, void *stream);
+
 /* The data movement around the convolutions (one HBM pass each; even grid
  * dimensions where a 2x level is involved).  Features: out[2][n][8] =
  * ((log10 K + 14)/2, conduit mask (NULL: 0), Dirichlet face mask +1 at x = 0

@@ -109,3 +109,46 @@ def test_wide_plane_grouped_forward(cin, cout):
                                b.double(), padding=1))
     assert _rel(ours, ref) < 6e-3
     guess.check_errors()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (33, 5, 2), (130, 3, 9), (32, 4, 40)])
+@pytest.mark.parametrize("cin,cout", sorted(guess._SHAPES))
+def test_weight_gradient_at_tile_edges(cin, cout, dims):
+    """Grids of one cell, ragged and full 32-cell columns, more z planes than
+    the kernel's ring; added into a gradient that is not 16-byte aligned."""
+    g = torch.Generator().manual_seed(cin * 11 + cout)
+    n = dims[0] * dims[1] * dims[2]
+    x = torch.randn(n, cin, generator=g).bfloat16()
+    dy = torch.randn(n, cout, generator=g).bfloat16()
+    xb, dyb = guess.blocked(x.cuda()), guess.blocked(dy.cuda())
+    buf = torch.ones(27 * cout * cin + 1, dtype=torch.float32, device="cuda")
+    dev = torch.device("cuda", torch.cuda.current_device())
+    rc = guess._lib().hmfem_conv3d_wgrad(
+        xb.data_ptr(), dyb.data_ptr(), buf.data_ptr() + 4, *dims, cin, cout,
+        guess._err_buf(dev).data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    ours = buf[1:].cpu().double().reshape(27, cout, cin) - 1.0
+    assert float(buf[0]) == 1.0
+    ref = torch.nn.grad.conv3d_weight(_to_ncdhw(x.double(), dims), (cout, cin, 3, 3, 3),
+                                      _to_ncdhw(dy.double(), dims), padding=1)
+    ref = ref.permute(2, 3, 4, 0, 1).reshape(27, cout, cin)
+    # exact BF16 products, FP32 sums, each added to a 1: 2^-24 per addition
+    assert float((ours - ref).abs().max()) < 1e-5 * (float(ref.abs().max()) + 1.0)
+    guess.check_errors()
+
+
+@pytest.mark.parametrize("n,slabs", [(1, 1), (1025, 2), (70001, 6)])
+def test_relu_and_bias_gradient(n, slabs):
+    g = torch.Generator().manual_seed(n)
+    gout = torch.randn(slabs, n, 8, generator=g).bfloat16().cuda()
+    out = torch.randn(slabs, n, 8, generator=g).relu().bfloat16().cuda()
+    ours, gb = guess.relu_grad_raw(gout, out)
+    ref = gout * (out > 0).to(gout.dtype)
+    assert torch.equal(ours.view(torch.int16), ref.view(torch.int16))
+    s = ref.double().sum(1).reshape(-1)
+    # FP32 partial sums: 2^-24 of the summed magnitude per addition
+    assert bool(((gb.double() - s).abs() <= 1e-6 * ref.double().abs().sum(1).reshape(-1)).all())
+    same, gb2 = guess.relu_grad_raw(gout, None)
+    assert same is gout
+    s = gout.double().sum(1).reshape(-1)
+    assert bool(((gb2.double() - s).abs() <= 1e-6 * gout.double().abs().sum(1).reshape(-1)).all())
