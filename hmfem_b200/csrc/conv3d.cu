@@ -192,6 +192,18 @@ __device__ __forceinline__ void tmem_wait_ld()
 // warps' lane quarters and, in plane mode, between consecutive runs of a z
 // plane).  Any other neighbour of a stored cell is a halo column, i.e. zero
 // padding, because the tile covers the whole x extent.
+// Grouped z taps (ZG, when 3 COUT <= 256 and a tile has at least 4 planes):
+// the three taps dz = -1, 0, +1 of a (dx, dy) pair share the operand of one
+// input plane zi and feed three output planes zi+1, zi, zi-1 at the same x
+// and y.  A run column's planes lie next to each other in tensor memory,
+// highest plane first, so one MMA with N = 3 COUT adds into all three at
+// once, and nothing has to be shifted afterwards.  The tile's first and last
+// planes take N = COUT and 2 COUT; a plane's first MMA (not accumulating) is
+// issued by itself.  9 (bz + 2) MMAs per run column and chunk instead of
+// 27 bz; each output still adds its taps in the order of the ungrouped form,
+// so its bits are the same.  Bound by the operands' shared-memory reads (44
+// cycles per MMA at COUT = 16).  Measured against the ungrouped and x-grouped
+// forms: see plan_conv.
 struct ConvPlan {
     int bx, by, bz;          // tile (interior cells)
     int W, H;                // halo row pitch bx+2, halo rows per plane by+2
@@ -202,6 +214,7 @@ struct ConvPlan {
     int ns, nb;              // input stages, accumulator buffers
     int wres;                // weights of every chunk resident
     int xg;                  // x taps grouped: N = 3 COUT per MMA (see k_conv3d)
+    int zg;                  // z taps grouped
     int tmem_cols;
     unsigned stage_bytes, wbytes, smem_bytes;
 };
@@ -232,6 +245,29 @@ __device__ __forceinline__ void umma_bf16_elect(uint32_t tmem, uint64_t da, uint
         "setp.ne.b32 p, %4, 0;\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
         "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+}
+
+// Eight accumulating MMAs into one accumulator, elected once: operand A at
+// da + off[i], operand B at db + (i + 1) BSTEP (16-byte units).
+template <int BSTEP>
+__device__ __forceinline__ void umma_bf16_elect8(uint32_t tmem, uint64_t da, const int off[8],
+                                                 uint64_t db, uint32_t idesc)
+{
+#define HM_MMA8_ONE(i, k)                                                               \
+    "add.s64 a, %1, %" #i ";\n\t"                                                       \
+    "add.s64 b, %2, %" #k ";\n\t"                                                       \
+    "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+    asm volatile(
+        "{\n\t.reg .pred e, p;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.eq.u32 p, %3, %3;\n\t" HM_MMA8_ONE(4, 12) HM_MMA8_ONE(5, 13) HM_MMA8_ONE(6, 14)
+            HM_MMA8_ONE(7, 15) HM_MMA8_ONE(8, 16) HM_MMA8_ONE(9, 17) HM_MMA8_ONE(10, 18)
+                HM_MMA8_ONE(11, 19) "}\n" ::"r"(tmem),
+        "l"(da), "l"(db), "r"(idesc), "l"((int64_t)off[0]), "l"((int64_t)off[1]),
+        "l"((int64_t)off[2]), "l"((int64_t)off[3]), "l"((int64_t)off[4]), "l"((int64_t)off[5]),
+        "l"((int64_t)off[6]), "l"((int64_t)off[7]), "n"(BSTEP), "n"(2 * BSTEP), "n"(3 * BSTEP),
+        "n"(4 * BSTEP), "n"(5 * BSTEP), "n"(6 * BSTEP), "n"(7 * BSTEP), "n"(8 * BSTEP));
+#undef HM_MMA8_ONE
 }
 
 __device__ __forceinline__ void umma_commit_elect(uint64_t *mbar)
@@ -281,6 +317,29 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1,
+                                            int c2, int c3, uint64_t *m)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(m))
+        : "memory");
+}
+
+// A position in a ring of barriers and the phase parity of its current use.
+struct Ring {
+    int i;
+    unsigned ph;
+    __device__ __forceinline__ void next(int n)
+    {
+        if (++i == n) {
+            i = 0;
+            ph ^= 1u;
+        }
+    }
+};
+
 // named barrier 1 among the epilogue warps; the reduction form returns the
 // AND of every thread's predicate (all threads agree on leaving)
 __device__ __forceinline__ void epi_sync()
@@ -329,14 +388,15 @@ __device__ __forceinline__ int run_start(const ConvPlan &p, int r, int &plane, i
     return 1 + p.W + p.W * p.H * (plane + 1) + 128 * (r - plane * p.rp);
 }
 
-template <int CIN, int COUT, bool XG>
+template <int CIN, int COUT, bool XG, bool ZG>
 __global__ void __launch_bounds__(kConvThreads, 1)
 k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorMap tm_w,
          const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out, int nx, int ny,
          int nz, int relu, const ConvPlan p, int *err)
 {
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 256, "channel counts");
-    static_assert(!XG || 3 * COUT <= 256, "grouped x taps: N = 3 COUT <= 256");
+    static_assert(!(XG || ZG) || 3 * COUT <= 256, "grouped taps: N = 3 COUT <= 256");
+    static_assert(!(XG && ZG), "one grouping at a time");
     constexpr int KC = CIN / 16;
     constexpr int NACC = XG ? 3 * COUT : COUT;  // accumulator columns per run
     constexpr uint32_t IDESC = idesc_bf16(128, NACC);
@@ -389,7 +449,10 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
         const int D = p.bz + 2, rows = p.H * D;
         unsigned wkc = 0xffffffffu;  // per stage (8 bits each): chunk of its weights
         long item = 0;
+        Ring ring{0, 0u};
         bool ok = true;
+        // row / H as a product: exact for row * H < 2^32
+        const unsigned inv_h = 0xffffffffu / (unsigned)p.H + 1u;
         for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
             const int tx = (int)(tile % p.ntx), ty = (int)((tile / p.ntx) % p.nty),
                       tz = (int)(tile / ((long)p.ntx * p.nty));
@@ -400,11 +463,10 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
             const int ya = y0 < 0 ? 0 : y0, yb = y0 + p.H < ny ? y0 + p.H : ny;
             const int za = z0 < 0 ? 0 : z0, zb = z0 + D < nz ? z0 + D : nz;
             const int rows_in = (yb - ya) * (zb - za);
-            for (int kc = 0; kc < KC; kc++, item++) {
-                const int s = (int)(item % p.ns);
-                const unsigned use = (unsigned)(item / p.ns);
+            for (int kc = 0; kc < KC; kc++, item++, ring.next(p.ns)) {
+                const int s = ring.i;
                 if (!__all_sync(0xffffffffu,
-                                role_wait(&empty[s], (use & 1u) ^ 1u, abort_flag, err))) {
+                                role_wait(&empty[s], ring.ph ^ 1u, abort_flag, err))) {
                     ok = false;
                     break;
                 }
@@ -418,8 +480,8 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
                 __syncwarp();
                 const uint4 zero = make_uint4(0, 0, 0, 0);
                 for (int i = lane; i < 2 * rows; i += 32) {
-                    const int sl = i / rows, rr = i - sl * rows, zi = rr / p.H,
-                              yi = rr - zi * p.H;
+                    const int sl = i >= rows, rr = i - sl * rows,
+                              zi = (int)__umulhi((unsigned)rr, inv_h), yi = rr - zi * p.H;
                     const int gy = y0 + yi, gz = z0 + zi;
                     unsigned char *drow_p = stages + (size_t)s * p.stage_bytes + (size_t)sl * SB +
                                             (size_t)(rr * p.W) * 16u;
@@ -439,8 +501,13 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
                     for (int c = p.wres ? 0 : kc; c < (p.wres ? KC : kc + 1); c++) {
                         const uint32_t wb = p.wres ? smem_u32(wres) + (uint32_t)c * 2u * WHALF
                                                    : a + SA;
-                        tma_load_3d(wb, &tm_w, 16 * c, 0, 0, &full[s]);
-                        tma_load_3d(wb + WHALF, &tm_w, 16 * c + 8, 0, 0, &full[s]);
+                        if (ZG) {  // [dx, dy][dz][COUT][8]
+                            tma_load_4d(wb, &tm_w, 16 * c, 0, 0, 0, &full[s]);
+                            tma_load_4d(wb + WHALF, &tm_w, 16 * c + 8, 0, 0, 0, &full[s]);
+                        } else {
+                            tma_load_3d(wb, &tm_w, 16 * c, 0, 0, &full[s]);
+                            tma_load_3d(wb + WHALF, &tm_w, 16 * c + 8, 0, 0, &full[s]);
+                        }
                     }
                 }
                 if (need_w) wkc = (wkc & ~(0xffu << (8 * s))) | ((unsigned)kc << (8 * s));
@@ -462,25 +529,26 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
         // per-tap offset held in a register, the B descriptor the stage's
         // base plus an immediate.
         {
-            constexpr int NT = XG ? 9 : 27;  // MMAs per run and chunk
+            constexpr int NT = XG || ZG ? 9 : 27;  // taps or groups of an operand run
             int offs[NT];
 #pragma unroll
             for (int t = 0; t < NT; t++)
-                offs[t] = XG ? p.W * (t % 3 - 1) + WH * (t / 3 - 1)
+                offs[t] = ZG   ? (t % 3 - 1) + p.W * (t / 3 - 1)
+                          : XG ? p.W * (t % 3 - 1) + WH * (t / 3 - 1)
                              : (t % 3 - 1) + p.W * ((t / 3) % 3 - 1) + WH * (t / 9 - 1);
-            long item = 0, jt = 0;
+            Ring ring{0, 0u}, acc_ring{0, 0u};
             bool ok = true;
-            for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, jt++) {
-                const int b = (int)(jt % p.nb);
-                const unsigned u = (unsigned)(jt / p.nb);
-                if (!__all_sync(0xffffffffu, role_wait(&tempty[b], (u & 1u) ^ 1u, abort_flag, err)))
+            for (long tile = blockIdx.x; tile < ntiles && ok;
+                 tile += gridDim.x, acc_ring.next(p.nb)) {
+                const int b = acc_ring.i;
+                if (!__all_sync(0xffffffffu,
+                                role_wait(&tempty[b], acc_ring.ph ^ 1u, abort_flag, err)))
                     break;
                 tc_after_sync();
                 const uint32_t acc0 = tmem + (uint32_t)(b * p.runs * NACC);
-                for (int kc = 0; kc < KC; kc++, item++) {
-                    const int s = (int)(item % p.ns);
-                    const unsigned use = (unsigned)(item / p.ns);
-                    if (!__all_sync(0xffffffffu, role_wait(&full[s], use & 1u, abort_flag, err))) {
+                for (int kc = 0; kc < KC; kc++, ring.next(p.ns)) {
+                    const int s = ring.i;
+                    if (!__all_sync(0xffffffffu, role_wait(&full[s], ring.ph, abort_flag, err))) {
                         ok = false;
                         break;
                     }
@@ -493,6 +561,38 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
                     const uint64_t da0 = kmajor_desc(a, SB, 128);
                     const uint64_t db0 = kmajor_desc(wb, WHALF, 128);
                     const uint32_t first = kc == 0 ? 0u : 1u;
+                    if (ZG) {
+                        for (int j = 0; j < p.rp; j++) {
+                            const uint64_t daj =
+                                da0 + (uint64_t)(1 + p.W * (p.row_mode ? j + 1 : 1) +
+                                                 (p.row_mode ? 0 : 128 * j));
+                            for (int zi = 0; zi < p.bz + 2; zi++) {
+                                // output planes zi - d, d = dz + 1 in [lo, hi]
+                                const int lo = zi < p.bz ? 0 : zi - p.bz + 1,
+                                          hi = zi < 2 ? zi : 2;
+                                const uint64_t dar = daj + (uint64_t)(WH * zi);
+                                const uint32_t acc =
+                                    acc0 + (uint32_t)((j * p.bz + p.bz - 1 - zi + lo) * COUT);
+                                const uint64_t db = db0 + (uint64_t)(lo * (WTAP / 16));
+                                const uint32_t idn = idesc_bf16(128, (hi - lo + 1) * COUT);
+                                // the plane that starts here (d = 0)
+                                const bool fresh = kc == 0 && zi < p.bz;
+                                if (fresh) {
+                                    umma_bf16_elect(acc, dar + (uint64_t)offs[0], db,
+                                                    idesc_bf16(128, COUT), 0u);
+                                    if (hi > 0)
+                                        umma_bf16_elect(acc + COUT, dar + (uint64_t)offs[0],
+                                                        db + (uint64_t)(WTAP / 16),
+                                                        idesc_bf16(128, hi * COUT), 1u);
+                                } else {
+                                    umma_bf16_elect(acc, dar + (uint64_t)offs[0], db, idn, 1u);
+                                }
+                                umma_bf16_elect8<3 * (WTAP / 16)>(acc, dar, offs + 1, db, idn);
+                            }
+                        }
+                        umma_commit_elect(&empty[s]);
+                        continue;
+                    }
                     // run starts without divisions (the order of run_start)
                     int plane = 0, j = 0;
                     for (int r = 0; r < p.runs; r++) {
@@ -542,8 +642,11 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
                 const bool v = zi == plane + 1 && yi >= 1 && yi <= p.by && xi >= 1 &&
                                xi <= p.bx && (row < 0 || yi == row + 1) && gx < nx && gy < ny &&
                                gz < nz;
+                // run r's columns: by run, or (grouped z taps) by run column,
+                // the highest plane first
+                const int rc = ZG ? (r - plane * p.rp) * p.bz + p.bz - 1 - plane : r;
                 const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) +
-                                    (uint32_t)((b * p.runs + r) * NACC);
+                                    (uint32_t)((b * p.runs + rc) * NACC);
                 const long cell = gx + (long)nx * (gy + (long)ny * gz);
                 // runs r-1 and r+1 of the same z plane (plane mode only)
                 const bool same_prev = !p.row_mode && r > 0 && r % p.rp != 0;
@@ -658,8 +761,8 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
 // taps in its columns: with 16 -> 16 channels 48 x 144 useful entries of
 // 128 x 144 for 16 cells, against 16 x 16 of 128 x 16 for one tap per MMA
 // (one tap per CTA, both operands transposed through registers).  Measured
-// against that form: 16 -> 16 at 128^3 2707 -> 136 us, 48 -> 16 3814 -> 262,
-// 96 -> 32 at 64^3 1335 -> 106, 64 -> 64 at 32^3 125 -> 32.  What bounds it
+// against that form: 16 -> 16 at 128^3 2707 -> 113 us, 48 -> 16 3814 -> 250,
+// 96 -> 32 at 64^3 1335 -> 104, 64 -> 64 at 32^3 125 -> 32.  What bounds it
 // now are the group copies (16 -> 16: 12 groups for each 128 x 144 MMA).
 //
 // A step is 32 x BY cells of one z plane.  A group is one slab (8 channels)
@@ -706,16 +809,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n)
     return idesc_bf16(m, n) | (1u << 15) | (1u << 16);
 }
 
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1,
-                                            int c2, int c3, uint64_t *m)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-        "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(m))
-        : "memory");
-}
-
 template <int NS, int BY>
 __global__ void __launch_bounds__(kConvThreads, 1)
 k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_n,
@@ -748,6 +841,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
     const uint32_t tmem = *tslot;
 
     if (warp == 4) {
+        Ring rm{0, 0u}, rn{0, 0u};
         long mseq = 0, nseq = 0;
         // this lane's group: of the M side (x shift, slab), of an N plane
         // (y shift, slab)
@@ -759,36 +853,34 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
                       zc = (int)(it / ((long)p.nxc * p.nyb));
             const int z0 = zc * p.zl, z1 = z0 + p.zl < nz ? z0 + p.zl : nz;
             for (int z = z0 - 1; z <= z1; z++) {  // N plane z, then M plane z - 1
-                const int sn = (int)(nseq % RN);
                 if (!__all_sync(0xffffffffu,
-                                role_wait(&empty_n[sn], ((unsigned)(nseq / RN) & 1u) ^ 1u,
-                                          abort_flag, err))) {
+                                role_wait(&empty_n[rn.i], rn.ph ^ 1u, abort_flag, err))) {
                     ok = false;
                     break;
                 }
-                if (lane == 0) mbar_expect_tx_only(&full_n[sn], GN * SP);
+                if (lane == 0) mbar_expect_tx_only(&full_n[rn.i], GN * SP);
                 __syncwarp();
                 if (lane < GN)
-                    tma_load_4d(smem_u32(nring + (sn * GN + lane) * SP), &tm_n, 256 * xc,
-                                BY * yb + nj - 1, z, nslab, &full_n[sn]);
+                    tma_load_4d(smem_u32(nring + (rn.i * GN + lane) * SP), &tm_n, 256 * xc,
+                                BY * yb + nj - 1, z, nslab, &full_n[rn.i]);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full_n[sn]);
+                if (lane == 0) mbar_arrive(&full_n[rn.i]);
+                rn.next(RN);
                 nseq++;
                 if (z <= z0) continue;
-                const int sm = (int)(mseq % RM);
                 if (!__all_sync(0xffffffffu,
-                                role_wait(&empty_m[sm], ((unsigned)(mseq / RM) & 1u) ^ 1u,
-                                          abort_flag, err))) {
+                                role_wait(&empty_m[rm.i], rm.ph ^ 1u, abort_flag, err))) {
                     ok = false;
                     break;
                 }
-                if (lane == 0) mbar_expect_tx_only(&full_m[sm], (uint32_t)(gmc * SP));
+                if (lane == 0) mbar_expect_tx_only(&full_m[rm.i], (uint32_t)(gmc * SP));
                 __syncwarp();
                 if (lane < gmc)
-                    tma_load_4d(smem_u32(mring + sm * mstage + lane * SP), &tm_m,
-                                256 * xc + 8 * (gi - 1), BY * yb, z - 1, gs, &full_m[sm]);
+                    tma_load_4d(smem_u32(mring + rm.i * mstage + lane * SP), &tm_m,
+                                256 * xc + 8 * (gi - 1), BY * yb, z - 1, gs, &full_m[rm.i]);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full_m[sm]);
+                if (lane == 0) mbar_arrive(&full_m[rm.i]);
+                rm.next(RM);
                 mseq++;
             }
         }
@@ -805,57 +897,66 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
         }
         __syncwarp();
     } else if (warp == 5) {
-        long mseq = 0, nseq = 0;
+        // ring positions kept incrementally: the scalar work between two
+        // steps' MMAs is this one warp's (positions from 64-bit remainders
+        // cost ~950 cycles a step)
+        Ring rm{0, 0u}, rn[3];  // planes z - 1, z, z + 1
+        for (int k = 0; k < 3; k++) rn[k] = Ring{k, 0u};
         bool ok = true;
         uint32_t acc = 0;  // nothing in D yet
-        const uint32_t nbase = smem_u32(nring), mbase = smem_u32(mring);
+        const uint64_t nbase = kmajor_desc(smem_u32(nring), 128, SP),
+                       mbase = kmajor_desc(smem_u32(mring), 128, SP);
         for (long it = idx; it < items && ok; it += p.per) {
             const int zc = (int)(it / ((long)p.nxc * p.nyb));
             const int z0 = zc * p.zl, z1 = z0 + p.zl < nz ? z0 + p.zl : nz;
-            for (int z = z0; z < z1 && ok; z++, nseq++, mseq++) {
-                // planes z - 1, z, z + 1 are ring items nseq .. nseq + 2
+            for (int z = z0; z < z1 && ok; z++) {
                 for (int k = z == z0 ? 0 : 2; k < 3; k++)
-                    ok = ok && __all_sync(0xffffffffu,
-                                          role_wait(&full_n[(nseq + k) % RN],
-                                                    (unsigned)((nseq + k) / RN) & 1u, abort_flag,
-                                                    err));
-                const int sm = (int)(mseq % RM);
-                ok = ok && __all_sync(0xffffffffu, role_wait(&full_m[sm],
-                                                             (unsigned)(mseq / RM) & 1u,
-                                                             abort_flag, err));
+                    ok = ok && __all_sync(0xffffffffu, role_wait(&full_n[rn[k].i], rn[k].ph,
+                                                                 abort_flag, err));
+                ok = ok && __all_sync(0xffffffffu,
+                                      role_wait(&full_m[rm.i], rm.ph, abort_flag, err));
                 if (!ok) break;
                 tc_after_sync();
-                const uint64_t da = kmajor_desc(mbase + (uint32_t)(sm * mstage), 128, SP);
-                const int r0 = (int)(nseq % RN);
+                const uint64_t da = mbase + (uint64_t)((rm.i * mstage) >> 4);
                 uint64_t db[3];
 #pragma unroll
                 for (int k = 0; k < 3; k++)
-                    db[k] = kmajor_desc(nbase + (uint32_t)(((nseq + k) % RN) * GN * SP), 128, SP);
+                    db[k] = nbase + (uint64_t)(rn[k].i * (GN * SP / 16));
                 // one MMA over the three planes where they are consecutive
                 // in the ring and N = 3 GN 8 <= 256, otherwise one per plane
-                const bool one = C::COLS <= 256 && r0 + 2 < RN;
+                if (C::COLS <= 256 && rn[0].i + 2 < RN) {
 #pragma unroll
-                for (int ks = 0; ks < C::KS; ks++) {
-                    const uint64_t o = (uint64_t)(16 * ks);  // 256 bytes
-                    if (one) {
-                        umma_bf16_elect(tmem, da + o, db[0] + o,
+                    for (int ks = 0; ks < C::KS; ks++) {  // 256 bytes further each
+                        umma_bf16_elect(tmem, da + (uint64_t)(16 * ks),
+                                        db[0] + (uint64_t)(16 * ks),
                                         idesc_bf16_mn(128, C::COLS <= 256 ? C::COLS : 256), acc);
-                    } else {
+                        acc = 1;
+                    }
+                } else {
+#pragma unroll
+                    for (int ks = 0; ks < C::KS; ks++) {
 #pragma unroll
                         for (int k = 0; k < 3; k++)
-                            umma_bf16_elect(tmem + (uint32_t)(k * GN * 8), da + o, db[k] + o,
+                            umma_bf16_elect(tmem + (uint32_t)(k * GN * 8),
+                                            da + (uint64_t)(16 * ks), db[k] + (uint64_t)(16 * ks),
                                             idesc_bf16_mn(128, GN * 8), acc);
+                        acc = 1;
                     }
-                    acc = 1;
                 }
-                umma_commit_elect(&empty_m[sm]);
-                umma_commit_elect(&empty_n[r0]);
+                umma_commit_elect(&empty_m[rm.i]);
+                umma_commit_elect(&empty_n[rn[0].i]);
                 if (z == z1 - 1) {  // the walk's last two planes
-                    umma_commit_elect(&empty_n[(nseq + 1) % RN]);
-                    umma_commit_elect(&empty_n[(nseq + 2) % RN]);
+                    umma_commit_elect(&empty_n[rn[1].i]);
+                    umma_commit_elect(&empty_n[rn[2].i]);
+                }
+                rm.next(RM);
+                // one plane on, or three at the end of the walk
+                for (int q = 0; q < (z == z1 - 1 ? 3 : 1); q++) {
+                    rn[0] = rn[1];
+                    rn[1] = rn[2];
+                    rn[2].next(RN);
                 }
             }
-            nseq += 2;
         }
         umma_commit_elect(done);
         if (lane == 0 && !mbar_wait(done, 0)) {
@@ -915,7 +1016,15 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
 // waves over the SMs -- subject to the tensor-memory columns (runs x COUT,
 // x3 grouped, doubled when two accumulators fit in 512) and the shared
 // memory.  Grouping pays where the MMAs dominate: many input chunks and
-// few output columns (48 -> 16 at 128^3: 255 -> 191 us).
+// few output columns, and the tile is too flat to group the z taps instead.
+// Grouping the z taps needs no work in the epilogue but two more input planes
+// per tile: from 4 planes on it halves the MMAs (at 2 planes it would save a
+// third of them and load twice the cells).  It adds an output's taps in the
+// order of the ungrouped form, the x grouping in another one: so z grouping
+// takes over from the ungrouped form only, and a shape's results keep their
+// bits.  Against the ungrouped form: 16 -> 16 at 128^3 95 -> 80 us, 32 -> 16
+// at 64^3 47 -> 36, 96 -> 32 100 -> 78; the copies of the halo rows (~55 us
+// alone at 16 -> 16) and the MMAs (~65 us) now bound it about equally.
 ConvPlan plan_conv(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_max)
 {
     ConvPlan best{};
@@ -924,17 +1033,19 @@ ConvPlan plan_conv(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_
     const unsigned wchunk = 27u * (unsigned)cout * 32u;
     // row mode (bx = 128, x tiles) when nx >= 128; plane mode (bx = nx, the
     // whole x extent) for any width up to kMaxPlaneX
+    for (int g = 0; g < 3 && !(g == 2 && best.xg); g++)
     for (int pm = 0; pm < 2; pm++)
-    for (int xg = 0; xg < 2; xg++)
         for (int bz = 1; bz <= (nz < 16 ? nz : 16); bz++)
             for (int by = 1; by <= (ny < 64 ? ny : 64); by++) {
                 const bool row_mode = pm == 0;
+                const int xg = g == 1, zg = g == 2;
                 if (row_mode ? nx < 128 : nx > kMaxPlaneX) continue;
                 const int bx = row_mode ? 128 : nx;
                 const int W = bx + 2;
                 // grouped x taps need N = 3 COUT <= 256 and tiles spanning
                 // the x extent (their x neighbours outside the tile are zero)
                 if (xg && (3 * cout > 256 || (row_mode && nx != 128))) continue;
+                if (zg && (3 * cout > 256 || bz < 4)) continue;
                 ConvPlan p{};
                 p.bx = bx;
                 p.by = by;
@@ -945,6 +1056,7 @@ ConvPlan plan_conv(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_
                 p.hcp = (p.hc + 128 + 7) / 8 * 8;
                 p.row_mode = row_mode;
                 p.xg = xg;
+                p.zg = zg;
                 p.rp = row_mode ? by : (W * (by - 1) + bx + 127) / 128;
                 p.runs = bz * p.rp;
                 const int nacc = (xg ? 3 : 1) * cout;
@@ -962,7 +1074,17 @@ ConvPlan plan_conv(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_
                 p.ntz = (nz + bz - 1) / bz;
                 const long tiles = (long)p.ntx * p.nty * p.ntz;
                 const double mma_c = nacc / 2.0 > 42.0 ? nacc / 2.0 : 42.0;
-                const double mma = (double)p.runs * (xg ? 9 : 27) * kc * mma_c;
+                double mma = (double)p.runs * (xg ? 9 : 27) * kc * mma_c;
+                if (zg) {  // per plane N = 1, 2, 3 .. 3, 2, 1 times COUT, and the first MMAs
+                    double c[4];
+                    for (int q = 1; q < 4; q++) {
+                        c[q] = q * cout / 2.0;                      // tensor pipe
+                        const double rd = (4096 + 32.0 * q * cout) / 128;  // operand reads
+                        if (c[q] < rd) c[q] = rd;
+                        if (c[q] < 42) c[q] = 42;
+                    }
+                    mma = p.rp * (kc * 9.0 * ((bz - 2) * c[3] + 2 * c[2] + 2 * c[1]) + bz * c[1]);
+                }
                 const double load = kc * (2.0 * p.H * (bz + 2) * 30.0 + 32.0 * p.hc / 48.0) +
                                     (p.wres ? 0.0 : 27.0 * cout * kc);
                 // epilogue per run and 16 columns (measured): ~300 cycles, ~2000
@@ -1036,10 +1158,21 @@ int launch_fwd(const void *in, const void *w, const float *bias, void *out, int 
     HM_CUDA(cudaGetDevice(&dev));
     HM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     HM_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const ConvPlan p = plan_conv(nx, ny, nz, CIN, COUT, nsm, smem_max);
-    auto k = k_conv3d<CIN, COUT, false>;
-    if constexpr (3 * COUT <= 256)
-        if (p.xg) k = k_conv3d<CIN, COUT, true>;
+    // the last plan this thread made for these channels: a network runs the
+    // same grid again and again, and the search takes some 50 us
+    struct Key { int nx, ny, nz, nsm, smem; };
+    static thread_local Key key{};
+    static thread_local ConvPlan plan;
+    if (key.nx != nx || key.ny != ny || key.nz != nz || key.nsm != nsm || key.smem != smem_max) {
+        plan = plan_conv(nx, ny, nz, CIN, COUT, nsm, smem_max);
+        key = {nx, ny, nz, nsm, smem_max};
+    }
+    const ConvPlan &p = plan;
+    auto k = k_conv3d<CIN, COUT, false, false>;
+    if constexpr (3 * COUT <= 256) {
+        if (p.xg) k = k_conv3d<CIN, COUT, true, false>;
+        if (p.zg) k = k_conv3d<CIN, COUT, false, true>;
+    }
     if (p.ns < 1) {
         set_last_error("conv3d: no tile fits in shared memory", __FILE__, __LINE__);
         return HMFEM_E_ARG;
@@ -1049,7 +1182,14 @@ int launch_fwd(const void *in, const void *w, const float *bias, void *out, int 
         return HMFEM_E_ARG;
     }
     CUtensorMap tm_w;
-    {
+    if (p.zg) {  // the taps as (dz, dx dy): dz inside
+        const cuuint64_t dims[4] = {(cuuint64_t)CIN, (cuuint64_t)COUT, 3, 9};
+        const cuuint64_t tap = (cuuint64_t)COUT * CIN * 2;
+        const cuuint64_t strides[3] = {(cuuint64_t)CIN * 2, 9 * tap, tap};
+        const cuuint32_t box[4] = {8, (cuuint32_t)COUT, 3, 9};
+        const int rc = encode_bf16_map(&tm_w, w, 4, dims, strides, box);
+        if (rc != HMFEM_OK) return rc;
+    } else {
         const cuuint64_t dims[3] = {(cuuint64_t)CIN, (cuuint64_t)COUT, 27};
         const cuuint64_t strides[2] = {(cuuint64_t)CIN * 2, (cuuint64_t)COUT * CIN * 2};
         const cuuint32_t box[3] = {8, (cuuint32_t)COUT, 27};

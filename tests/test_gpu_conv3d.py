@@ -152,3 +152,20 @@ def test_relu_and_bias_gradient(n, slabs):
     assert same is gout
     s = gout.double().sum(1).reshape(-1)
     assert bool(((gb2.double() - s).abs() <= 1e-6 * gout.double().abs().sum(1).reshape(-1)).all())
+
+
+@pytest.mark.parametrize("dims", [(128, 3, 9), (40, 5, 4), (17, 16, 6), (64, 7, 21), (130, 2, 11),
+                                  (8, 8, 32)])
+@pytest.mark.parametrize("cin,cout", sorted(guess._SHAPES))
+def test_forward_exact_on_integers(cin, cout, dims):
+    """Small integers: every sum is exact in FP32, so the output is the
+    BF16 rounding of the exact value, whatever taps share an MMA."""
+    g = torch.Generator().manual_seed(cin + 3 * cout)
+    n = dims[0] * dims[1] * dims[2]
+    x = torch.randint(-4, 5, (n, cin), generator=g).bfloat16()
+    w = torch.randint(-3, 4, (27, cout, cin), generator=g).bfloat16()
+    b = torch.randint(-8, 9, (cout,), generator=g).float()
+    ref = _from_ncdhw(F.conv3d(_to_ncdhw(x.double(), dims), _w_torch(w.double()), b.double(),
+                               padding=1))
+    assert torch.equal(_fwd(x, w, b, dims, False), ref.float().bfloat16().double())
+    guess.check_errors()
