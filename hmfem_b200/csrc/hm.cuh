@@ -97,6 +97,9 @@ struct Level {
     float *pw32 = nullptr;
     Csr R;                    // P^T rows: fine ids ascending
     bool p_deferred = false;  // P not formed (level 0 of the exact reduction)
+    // made by amg_tail: the transfer (sel, cid, P, R, weights) and the matrix
+    // (A, dinv) lie in the solver's arena and are not freed one by one
+    bool tail_transfer = false, tail_matrix = false;
     int *cpts = nullptr;      // 19-offset level: the row of each coarse row (setup)
     // V-cycle vectors (FP64 and FP32 sets)
     double *f = nullptr, *ua = nullptr, *ub = nullptr, *rs = nullptr;
@@ -171,6 +174,15 @@ int launch_spmv(const Sell &S, const double *x, double *y, cudaStream_t st);
 // (rap_stencil.cu), bit-identical to the generic kernels.
 int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *err_dev,
                 const int *grid3 = nullptr, bool schur = false);
+// the rest of the hierarchy below level l >= 1 of at most 512 rows, in one
+// launch (amg_tail.cu): appends the levels to lv, *levels of them (0: the
+// general path has to go on)
+struct TailArena {
+    unsigned char *mem = nullptr;  // kept by the solver; what setup made lies here
+};
+bool tail_applies(const Level &L, int l);
+int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, TailArena &T,
+             cudaStream_t st, int *levels);
 // the reference's P of a level whose setup left it out (p_deferred)
 int ensure_p(Level &L, cudaStream_t st);
 int stencil_parity_split(int nx, int ny, int nz, signed char *sel, cudaStream_t st);
