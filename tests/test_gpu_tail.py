@@ -74,3 +74,33 @@ def test_coarse_inverse_solves(n):
     ref = np.linalg.solve(A, f)
     assert np.abs(u - ref).max() <= 1e-13 * (n * n + 10) * np.abs(ref).max()
     s.close()
+
+
+@pytest.mark.parametrize("n,band", [(1023, 3), (1024, 40), (1025, 90), (2500, 70), (3000, 200)])
+def test_greedy_split_of_banded_matrices(n, band):
+    """The general split around its 1024-row tiles, with rows shorter and
+    longer than the 64 entries its masks cover: every level the oracle's."""
+    rng = np.random.default_rng(n + band)
+    up = [np.unique(i + 1 + rng.integers(0, 2 * band, band)) for i in range(n)]
+    rows = [dict() for _ in range(n)]
+    for i, js in enumerate(up):
+        for j in js[js < n]:
+            rows[i][int(j)] = rows[int(j)][i] = -float(rng.random() + 0.1)
+    cnt, col, ele = np.zeros(n, np.int32), [], []
+    for i, r in enumerate(rows):
+        r[i] = 1.0 - sum(r.values())
+        cnt[i] = len(r)
+        for j in sorted(r):
+            col.append(j)
+            ele.append(r[j])
+    col, ele = np.array(col, np.int32), np.array(ele)
+    H = Port().amg(cnt, col, ele)
+    s = gpu.Solver()
+    s.set_matrix(cnt, col, ele)
+    s.setup()
+    assert s.num_levels() == H.nlevels
+    for l in range(H.nlevels):
+        g, o = s.level(l), H.level(l)
+        for k in ("cnt", "col", "ele", "sel", "pcnt", "pcol")[:3 if l == H.nlevels - 1 else 6]:
+            assert np.array_equal(g[k], o[k]), (l, k)
+    s.close()
