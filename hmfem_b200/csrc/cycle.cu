@@ -880,6 +880,11 @@ static int cycle_t(Solver &s, int l, cudaStream_t st, bool dot, bool seeded)
         HM_LAUNCHED();
         return HMFEM_OK;
     }
+    // from here down in one launch, where the levels fit
+    if (l == s.small.first && (s.small.kind == 0) == std::is_same<T, double>::value && seeded) {
+        const ChebCoef cc = cheb_coef(s.opt.cheb_degree);
+        return small_cycle(s, cc.c1, cc.c2, cc.ith, ctl, st);
+    }
     if (l == last) {
         launch_pdl(k_diag_solve<T>, nb(n), 256, st, n, s.vec_dtrue<T>(l), f, ua, ctl);
         HM_LAUNCHED();

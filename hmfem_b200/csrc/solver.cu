@@ -263,6 +263,7 @@ static void free_hierarchy(Solver &s, bool keep_l0)
     dfree(s.dense_L);
     s.dense_L = nullptr;
     s.direct_level = -1;
+    s.small.first = -1;
     s.nlevels = s.lv.size();
     s.setup_done = false;
     s.schur0_built = false;
@@ -524,6 +525,7 @@ int setup(Solver &s)
         }
         HM_PHASE("setup: colouring", st);
     }
+    HM_CHECK(small_cycle_build(s, st));
     int nonpos = 0;
     HM_CUDA(cudaMemcpyAsync(&nonpos, s.dwork + 8, sizeof(int), cudaMemcpyDeviceToHost, st));
     HM_CUDA(cudaStreamSynchronize(st));
@@ -956,6 +958,7 @@ int hmfem_destroy(hmfem_solver *h)
     hm::dfree(s.ctl); hm::dfree(s.part); hm::dfree(s.dwork); hm::dfree(s.mm);
     hm::dfree(s.gsbar);
     hm::dfree(s.tail.mem);
+    hm::dfree(s.small.masks);
     hm::alloc_cache_release(s.cache);
     s.cache = nullptr;
     hm::set_alloc_context(s.st, nullptr);

@@ -10,6 +10,28 @@ namespace hm {
 template <class T> struct Seed;  // cycle.cuh
 struct Demote;                     // cycle.cuh
 
+// The coarse end of the V-cycle in one launch (small_cycle.cu): the levels
+// from `first` to the coarse solve, each CTA's shared-memory layout.
+constexpr int kScLevels = 6, kScCtas = 16;
+struct SmallLayout {
+    struct Lv {
+        int own, cown;
+        unsigned o_val, o_col, o_slice, o_prow, o_pcol, o_rrow, o_rcol, o_f, o_u, o_r, o_dv,
+            o_b[2];
+        int at[kScCtas + 1][3];
+    } lv[kScLevels];
+    unsigned o_df, o_du, o_dense;
+
+};
+struct SmallCycle {
+    int first = -1;  // -1: not in use
+    int ctas = 0, kind = 0;
+    size_t smem = 0;
+    SmallLayout layout{};
+    int mask0 = 0;              // the first level's entry of
+    unsigned *masks = nullptr;  // which CTAs read a CTA's rows; kept by the solver
+};
+
 struct Solver {
     hmfem_options opt;
     cudaStream_t st = nullptr;
@@ -47,6 +69,7 @@ struct Solver {
     Ctl *ctl_host = nullptr;  // pinned, 2 slots
     double *part = nullptr;
     int *dwork = nullptr;
+    SmallCycle small;
     TailArena tail;        // the small levels' arrays (amg_tail.cu)
     unsigned *gsbar = nullptr;  // grid barrier of the fused Gauss-Seidel sweeps
     bool ctl_active = false;
@@ -103,6 +126,9 @@ int launch_smoother_diag(const Csr &A, int kind, double *dsm, float *dsm32,
                          cudaStream_t st);
 int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st);
 int time_kernel(Solver &s, int which, int l, int reps, float *ms, double *bytes);
+int small_cycle_build(Solver &s, cudaStream_t st);
+int small_cycle(Solver &s, const double *c1, const double *c2, double ith, const Ctl *ctl,
+                cudaStream_t st);
 int level_spmv(Solver &s, int l, const double *x, double *y, cudaStream_t st);
 
 // structured level-0 / level-1 kernels (stencil_cycle.cu); V is the
