@@ -22,6 +22,7 @@
 
 #include "grid19.cuh"
 #include <stdlib.h>
+#include <string.h>
 
 #include "hm.cuh"
 
@@ -216,8 +217,10 @@ struct UnionArgs {
     const int *orow, *ocol;  // outer rows: stage 0 A, stage 1 R
     const double *oval;      // stage 0: A values
     const double *w;         // P weight per fine row
-    const int *irow, *icol;  // inner rows: stage 0 P, stage 1 AP
-    const double *ival;      // stage 1: AP values
+    const int *irow, *icol;  // inner rows: stage 0 P (row pointers), stage 1 AP
+    const double *ival;      // stage 1: AP values,
+    const long long *iptr;   // its padded rows' starts and lengths
+    const int *ilen;
     const long long *cptr;   // candidate offsets (pass A scan)
     int *ucnt;               // distinct columns per row
     int *pcol;               // padded output
@@ -226,6 +229,18 @@ struct UnionArgs {
     int *err;
 };
 
+// inner row j: its first entry and length
+template <int STAGE>
+__device__ __forceinline__ long long inner_at(const UnionArgs &A, int j)
+{
+    return STAGE == 0 ? (long long)A.irow[j] : A.iptr[j];
+}
+template <int STAGE>
+__device__ __forceinline__ int inner_len(const UnionArgs &A, int j)
+{
+    return STAGE == 0 ? A.irow[j + 1] - A.irow[j] : A.ilen[j];
+}
+
 template <int STAGE>
 __global__ void k_cand_count(UnionArgs A, long long *ccnt)
 {
@@ -233,8 +248,7 @@ __global__ void k_cand_count(UnionArgs A, long long *ccnt)
          r += (long)gridDim.x * blockDim.x) {
         long long m = 0;
         for (int k = A.orow[r]; k < A.orow[r + 1]; k++) {
-            int j = A.ocol[k];
-            m += A.irow[j + 1] - A.irow[j];
+            m += inner_len<STAGE>(A, A.ocol[k]);
         }
         ccnt[r] = m;
     }
@@ -273,8 +287,8 @@ __device__ void gen_row(const UnionArgs &A, int r, unsigned long long *keys,
         int k = c0 + gr;
         bool ok = k < oe;
         int j = ok ? A.ocol[k] : 0;
-        int ib = ok ? A.irow[j] : 0;
-        int len = ok ? A.irow[j + 1] - ib : 0;
+        const long long ib = ok ? inner_at<STAGE>(A, j) : 0;
+        int len = ok ? inner_len<STAGE>(A, j) : 0;
         double s = 0.0;
         if (ok) s = STAGE == 0 ? dmul(A.oval[k], A.w[j]) : A.w[j];
         // exclusive scan of len over the group
@@ -382,22 +396,24 @@ k_union_warp(UnionArgs A, const int *rows, const int *nrows_dev, int tier)
 // distinct count passes HCAP/2 is abandoned (nothing written yet) and goes
 // to list[tier]; as at most 32 keys enter per chunk, the load stays below
 // HCAP - 32 and every probe sequence ends.
+template <int HCAP>
+struct HashMem {
+    int key[HCAP];
+    double val[HCAP];
+    unsigned long long sorted[HCAP / 2];
+    double cv[32];
+    long long ib[32];
+    double sc[32];
+    int off[34];
+};
+
 template <int STAGE, int HCAP>
 __global__ void __launch_bounds__(128)
 k_union_hash(UnionArgs A, const int *rows, const int *nrows_dev, int tier)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    struct WarpMem {
-        int key[HCAP];
-        double val[HCAP];
-        unsigned long long sorted[HCAP / 2];
-        double cv[32];
-        int off[33], ib[32];
-        double sc[32];
-    };
-    static_assert(sizeof(WarpMem) % 8 == 0, "alignment");
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpMem &M = ((WarpMem *)s_raw)[w];
+    HashMem<HCAP> &M = ((HashMem<HCAP> *)s_raw)[w];
     const long nr = rows ? *nrows_dev : A.nrows;
     for (long t = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; t < nr;
          t += ((long)gridDim.x * blockDim.x) >> 5) {
@@ -413,8 +429,8 @@ k_union_hash(UnionArgs A, const int *rows, const int *nrows_dev, int tier)
             const int k = c0 + lane;
             const bool ok = k < oe;
             const int j = ok ? A.ocol[k] : 0;
-            const int ib = ok ? A.irow[j] : 0;
-            const int len = ok ? A.irow[j + 1] - ib : 0;
+            const long long ib = ok ? inner_at<STAGE>(A, j) : 0;
+            const int len = ok ? inner_len<STAGE>(A, j) : 0;
             double sc = 0.0;
             if (ok) sc = STAGE == 0 ? dmul(A.oval[k], A.w[j]) : A.w[j];
             int x = len;
@@ -439,7 +455,7 @@ k_union_hash(UnionArgs A, const int *rows, const int *nrows_dev, int tier)
                         int mid = (lo + hi + 1) >> 1;
                         if (M.off[mid] <= g) lo = mid; else hi = mid - 1;
                     }
-                    const int q = M.ib[lo] + (g - M.off[lo]);
+                    const long long q = M.ib[lo] + (g - M.off[lo]);
                     col = A.icol[q];
                     // stage 0: a_ij * p_jd (= w_j); stage 1: AP[i][d] * w_i
                     tv = STAGE == 0 ? M.sc[lo] : dmul(A.ival[q], M.sc[lo]);
@@ -501,13 +517,6 @@ k_union_hash(UnionArgs A, const int *rows, const int *nrows_dev, int tier)
     }
 }
 
-template <int STAGE, int HCAP>
-size_t hash_smem()
-{
-    return 4 * (sizeof(int) * HCAP + sizeof(double) * HCAP + 8 * (HCAP / 2) +
-                8 * 32 + 4 * 33 + 4 * 32 + 8 * 32 + 4);
-}
-
 // Block per row for the longest rows (dynamic shared memory, cap entries).
 template <int STAGE>
 __global__ void __launch_bounds__(256)
@@ -565,53 +574,58 @@ int nblk(long n, int threads, long cap = 148L * 16)
     return (int)(b < cap ? b : cap);
 }
 
-// Runs passes A-C of one Galerkin stage into `out`.
+// Pass A of one Galerkin stage: candidate offsets; their total is read back
+// into PIN_CAND (two words).
 template <int STAGE>
-int run_union(UnionArgs A, Csr &out, int *dwork, cudaStream_t st)
+int union_count(const UnionArgs &A, long long *cptr, cudaStream_t st)
 {
     const int n = A.nrows;
-    out.n = n;
-    long long *cptr = (long long *)dalloc(sizeof(long long) * (n + 1));
-    out.rowptr = (int *)dalloc(sizeof(int) * (n + 1));
-    int *lists = (int *)dalloc(sizeof(int) * 2 * (n > 0 ? n : 1));
-    if (!cptr || !out.rowptr || !lists) {
-        set_last_error("out of device memory (RAP)", __FILE__, __LINE__);
-        return HMFEM_E_CUDA;
-    }
-    // pass A
     k_cand_count<STAGE><<<nblk(n, 256), 256, 0, st>>>(A, cptr);
     HM_LAUNCHED();
     HM_CUDA(cudaMemsetAsync(cptr + n, 0, sizeof(long long), st));
-    {
-        size_t tmp = 0;
-        HM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, cptr, cptr, n + 1, st));
-        void *t = dalloc(tmp);
-        HM_CUDA(cub::DeviceScan::ExclusiveSum(t, tmp, cptr, cptr, n + 1, st));
-        dfree(t);
-    }
-    long long mtot = 0;
-    HM_CUDA(cudaMemcpyAsync(&mtot, cptr + n, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-    A.cptr = cptr;
-    A.pcol = (int *)dalloc(sizeof(int) * (mtot > 0 ? mtot : 1));
-    A.pval = (double *)dalloc(sizeof(double) * (mtot > 0 ? mtot : 1));
-    if (!A.pcol || !A.pval) {
+    size_t tmp = 0;
+    HM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, cptr, cptr, n + 1, st));
+    void *t = dalloc(tmp);
+    if (!t) return HMFEM_E_CUDA;
+    HM_CUDA(cub::DeviceScan::ExclusiveSum(t, tmp, cptr, cptr, n + 1, st));
+    dfree(t);
+    return read_back(PIN_CAND, cptr + n, 2, st);
+}
+
+long long union_candidates()
+{
+    long long m = 0;
+    memcpy(&m, pinned_words() + PIN_CAND, sizeof(m));
+    return m;
+}
+
+// Pass B: distinct columns and sums of every row at A.cptr's padded place,
+// the rows' lengths in A.ucnt; an error flag is read back into err_slot.
+template <int STAGE>
+int union_rows(UnionArgs &A, int err_slot, int *dwork, cudaStream_t st)
+{
+    const int n = A.nrows;
+    int *lists = (int *)dalloc(sizeof(int) * 2 * (n > 0 ? n : 1));
+    const long long m = union_candidates();
+    A.pcol = (int *)dalloc(sizeof(int) * (m > 0 ? m : 1));
+    A.pval = (double *)dalloc(sizeof(double) * (m > 0 ? m : 1));
+    if (!lists || !A.pcol || !A.pval) {
         set_last_error("out of device memory (RAP)", __FILE__, __LINE__);
         return HMFEM_E_CUDA;
     }
-    A.ucnt = out.rowptr;
     A.list[0] = lists;
     A.list[1] = lists + n;
     A.nlist[0] = dwork;
     A.nlist[1] = dwork + 1;
     A.err = dwork + 2;
     HM_CUDA(cudaMemsetAsync(dwork, 0, 3 * sizeof(int), st));
-    // pass B: three tiers (<= 64 distinct columns, <= 512, <= 4096
-    // candidates)
+    // (a row over the last tier's capacity stays empty, and err is set)
+    HM_CUDA(cudaMemsetAsync(A.ucnt, 0, sizeof(int) * (n > 0 ? n : 1), st));
+    // three tiers (<= 64 distinct columns, <= 512, <= 4096 candidates)
     {
         auto k0 = k_union_hash<STAGE, 128>;
         auto k1 = k_union_hash<STAGE, 1024>;
-        const size_t m0 = hash_smem<STAGE, 128>(), m1 = hash_smem<STAGE, 1024>();
+        const size_t m0 = 4 * sizeof(HashMem<128>), m1 = 4 * sizeof(HashMem<1024>);
         HM_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m0));
         HM_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m1));
         k0<<<nblk((long)n * 32, 128, 148L * 64), 128, m0, st>>>(A, nullptr, nullptr, 0);
@@ -625,37 +639,18 @@ int run_union(UnionArgs A, Csr &out, int *dwork, cudaStream_t st)
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm));
     k_union_block<STAGE><<<148 * 2, 256, bsm, st>>>(A, A.list[1], A.nlist[1], bcap);
     HM_LAUNCHED();
-    // pass C
-    HM_CHECK(rowptr_from_counts(out.rowptr, n, st, &out.nnz));
-    int herr = 0;
-    HM_CUDA(cudaMemcpyAsync(&herr, A.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-    if (herr) {
-        set_last_error("sparse row over the Galerkin-product capacity", __FILE__, __LINE__);
-        return HMFEM_E_CAPACITY;
-    }
-    out.col = (int *)dalloc(sizeof(int) * (out.nnz > 0 ? out.nnz : 1));
-    out.val = (double *)dalloc(sizeof(double) * (out.nnz > 0 ? out.nnz : 1));
-    if (!out.col || !out.val) {
-        set_last_error("out of device memory (RAP)", __FILE__, __LINE__);
-        return HMFEM_E_CUDA;
-    }
-    k_compact<<<nblk((long)n * 32, 256, 148L * 32), 256, 0, st>>>(
-        cptr, out.rowptr, n, A.pcol, A.pval, out.col, out.val);
-    HM_LAUNCHED();
-    dfree(A.pcol);
-    dfree(A.pval);
-    dfree(cptr);
     dfree(lists);
-    return HMFEM_OK;
+    return read_back(err_slot, A.err, 1, st);
 }
 
-}  // namespace
+int union_error(int slot)
+{
+    if (!pinned_words()[slot]) return HMFEM_OK;
+    set_last_error("sparse row over the Galerkin-product capacity", __FILE__, __LINE__);
+    return HMFEM_E_CAPACITY;
+}
 
-// P rows (amg.h:332-346), their entries (amg.h:352-380) and weights from
-// the level's split and coarse ids; *pown: the fine row of every entry
-// (for the transpose), freed by the caller, or nullptr not to keep it.
-int build_p(Level &L, cudaStream_t st, int **pown_out)
+int p_count(Level &L, cudaStream_t st)
 {
     const int n = L.A.n;
     L.P.n = n;
@@ -663,7 +658,12 @@ int build_p(Level &L, cudaStream_t st, int **pown_out)
     if (!L.P.rowptr) return HMFEM_E_CUDA;
     k_pcount<<<nblk(n, 256), 256, 0, st>>>(L.A.rowptr, L.A.col, L.sel, n, L.P.rowptr);
     HM_LAUNCHED();
-    HM_CHECK(rowptr_from_counts(L.P.rowptr, n, st, &L.P.nnz));
+    return rowptr_scan(L.P.rowptr, n, st);
+}
+
+int p_fill(Level &L, cudaStream_t st, int **pown_out)
+{
+    const int n = L.A.n;
     L.P.col = (int *)dalloc(sizeof(int) * (L.P.nnz > 0 ? L.P.nnz : 1));
     int *pown = (int *)dalloc(sizeof(int) * (L.P.nnz > 0 ? L.P.nnz : 1));
     L.pw = (double *)dalloc(sizeof(double) * (n > 0 ? n : 1));
@@ -682,10 +682,46 @@ int build_p(Level &L, cudaStream_t st, int **pown_out)
     return HMFEM_OK;
 }
 
+// R = P^T by a stable radix sort on the coarse id (fine rows stay ascending)
+int r_sort(Level &L, const int *pown, cudaStream_t st)
+{
+    int *keys_out = (int *)dalloc(sizeof(int) * (L.P.nnz > 0 ? L.P.nnz : 1));
+    if (!keys_out) return HMFEM_E_CUDA;
+    HM_CUDA(cudaMemsetAsync(L.R.rowptr, 0, sizeof(int) * (L.nc + 1), st));
+    k_hist<<<nblk(L.P.nnz, 256), 256, 0, st>>>(L.P.col, L.P.nnz, L.R.rowptr);
+    HM_LAUNCHED();
+    HM_CHECK(rowptr_scan(L.R.rowptr, L.nc, st));
+    size_t tmp = 0;
+    int bits = 1;
+    while ((1l << bits) < (long)L.nc + 1) bits++;
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, L.P.col, keys_out, pown, L.R.col,
+                                            (int)L.P.nnz, 0, bits, st));
+    void *t = dalloc(tmp);
+    if (!t) return HMFEM_E_CUDA;
+    HM_CUDA(cub::DeviceRadixSort::SortPairs(t, tmp, L.P.col, keys_out, pown, L.R.col,
+                                            (int)L.P.nnz, 0, bits, st));
+    dfree(t);
+    dfree(keys_out);
+    return HMFEM_OK;
+}
+
+}  // namespace
+
+// P rows (amg.h:332-346), their entries (amg.h:352-380) and weights from
+// the level's split and coarse ids.
+static int build_p(Level &L, cudaStream_t st)
+{
+    HM_CHECK(p_count(L, st));
+    HM_CHECK(read_back(PIN_P, L.P.rowptr + L.A.n, 1, st));
+    HM_CUDA(cudaStreamSynchronize(st));
+    HM_CHECK(rowptr_total(PIN_P, &L.P.nnz));
+    return p_fill(L, st, nullptr);
+}
+
 int ensure_p(Level &L, cudaStream_t st)
 {
     if (!L.p_deferred) return HMFEM_OK;
-    HM_CHECK(build_p(L, st, nullptr));
+    HM_CHECK(build_p(L, st));
     HM_CUDA(cudaStreamSynchronize(st));
     return HMFEM_OK;
 }
@@ -747,25 +783,49 @@ int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *dwork,
             HM_LAUNCHED();
         }
     }
-    int herr[2] = {0, 0};
-    HM_CUDA(cudaMemcpyAsync(&herr[0], dwork, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (wave_err)
-        HM_CUDA(cudaMemcpyAsync(&herr[1], wave_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-    dfree(wave);
-    HM_PHASE("  C/F split", st);
-    if (herr[0] || herr[1]) {
-        set_last_error("C/F split wavefront gave up waiting", __FILE__, __LINE__);
-        return HMFEM_E_TIMEOUT;
-    }
+    HM_CHECK(read_back(PIN_ERR, dwork, 1, st));
+    if (wave_err) HM_CHECK(read_back(PIN_ERR2, wave_err, 1, st));
+    else pinned_words()[PIN_ERR2] = 0;
     // ---- coarse numbering ---------------------------------------------
     L.cid = (int *)dalloc(sizeof(int) * (n + 1));
+    if (!L.cid) return HMFEM_E_CUDA;
     k_cflag<<<nblk(n, 256), 256, 0, st>>>(L.sel, n, L.cid);
     HM_LAUNCHED();
-    long nc = 0;
-    HM_CHECK(rowptr_from_counts(L.cid, n, st, &nc));
-    HM_PHASE("  coarse ids", st);
-    L.nc = (int)nc;
+    HM_CHECK(rowptr_scan(L.cid, n, st));
+    // ---- P rows and, for the general product, the candidates of A P -------
+    // (all of this level's sizes are read back at once; a grid's are known)
+    const bool g19 = L.g19.nx > 0, general = !grid3 && !g19;
+    long long *cptr0 = nullptr;
+    UnionArgs a0{};
+    a0.nrows = n;
+    a0.orow = L.A.rowptr; a0.ocol = L.A.col; a0.oval = L.A.val;
+    if (!(grid3 && schur)) HM_CHECK(p_count(L, st));
+    if (grid3) {
+        L.nc = (int)parity_coarse(grid3[0], grid3[1], grid3[2]);
+        if (!schur) L.P.nnz = parity_pnnz(grid3[0], grid3[1], grid3[2]);
+    } else {
+        HM_CHECK(read_back(PIN_NC, L.cid + n, 1, st));
+        HM_CHECK(read_back(PIN_P, L.P.rowptr + n, 1, st));
+        if (general) {
+            cptr0 = (long long *)dalloc(sizeof(long long) * ((long)n + 1));
+            if (!cptr0) return HMFEM_E_CUDA;
+            a0.irow = L.P.rowptr;
+            HM_CHECK(union_count<0>(a0, cptr0, st));
+        }
+        HM_CUDA(cudaStreamSynchronize(st));
+        dfree(wave);
+        HM_PHASE("  C/F split and sizes", st);
+        if (pinned_words()[PIN_ERR] || pinned_words()[PIN_ERR2]) {
+            dfree(cptr0);
+            set_last_error("C/F split wavefront gave up waiting", __FILE__, __LINE__);
+            return HMFEM_E_TIMEOUT;
+        }
+        long t = 0;
+        HM_CHECK(rowptr_total(PIN_NC, &t));
+        L.nc = (int)t;
+        HM_CHECK(rowptr_total(PIN_P, &L.P.nnz));
+    }
+    const long nc = L.nc;
     // the next level's split from the 19-offset structure, on the side
     // stream, overlapping the rest of this level's coarsening
     if (grid3 && g19_applies(grid3[0], grid3[1], grid3[2]) && nc > 0) {
@@ -795,42 +855,25 @@ int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *dwork,
         L.p_deferred = true;
     } else {
         int *pown = nullptr;
-        HM_CHECK(build_p(L, st, &pown));
+        HM_CHECK(p_fill(L, st, &pown));
         L.R.n = L.nc;
         L.R.nnz = L.P.nnz;
         L.R.rowptr = (int *)dalloc(sizeof(int) * (L.nc + 1));
         L.R.col = (int *)dalloc(sizeof(int) * (L.P.nnz > 0 ? L.P.nnz : 1));
+        if (!L.R.rowptr || !L.R.col) return HMFEM_E_CUDA;
         bool done = false;
         if (grid3) {
             HM_CHECK(stencil_parity_R(grid3[0], grid3[1], grid3[2], L.cid, L.nc, L.R, st));
             done = true;
-        } else if (L.g19.nx > 0) {
-            HM_CHECK(g19_transpose(L, L.R, st, &done));
-        }
-        if (done) {
-            dfree(pown);
-        } else {  // stable radix sort on the coarse id
-            int *keys_out = (int *)dalloc(sizeof(int) * (L.P.nnz > 0 ? L.P.nnz : 1));
-            HM_CUDA(cudaMemsetAsync(L.R.rowptr, 0, sizeof(int) * (L.nc + 1), st));
-            k_hist<<<nblk(L.P.nnz, 256), 256, 0, st>>>(L.P.col, L.P.nnz, L.R.rowptr);
-            HM_LAUNCHED();
-            long rn = 0;
-            HM_CHECK(rowptr_from_counts(L.R.rowptr, L.nc, st, &rn));
-            size_t tmp = 0;
-            int bits = 1;
-            while ((1l << bits) < (long)L.nc + 1) bits++;
-            HM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, L.P.col, keys_out,
-                                                    pown, L.R.col, (int)L.P.nnz, 0,
-                                                    bits, st));
-            void *t = dalloc(tmp);
-            HM_CUDA(cub::DeviceRadixSort::SortPairs(t, tmp, L.P.col, keys_out, pown,
-                                                    L.R.col, (int)L.P.nnz, 0, bits,
-                                                    st));
+        } else if (g19_has_structure(L) && L.nc > 0) {
+            HM_CHECK(g19_transpose_rows(L, L.R, dwork, st));
             HM_CUDA(cudaStreamSynchronize(st));
-            dfree(t);
-            dfree(keys_out);
-            dfree(pown);
+            // (otherwise not this structure: the sort forms R)
+            done = !pinned_words()[PIN_RBAD] && pinned_words()[PIN_R] == L.P.nnz;
+            if (done) HM_CHECK(g19_transpose_fill(L, L.R, st));
         }
+        if (!done) HM_CHECK(r_sort(L, pown, st));
+        dfree(pown);
     }
     if (L.g19.nx > 0) HM_CHECK(g19_cpts(L, st));  // for the product
     HM_PHASE("  P and R", st);
@@ -847,6 +890,10 @@ int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *dwork,
             C.g19.nz = grid3[2];
             C.g19.v = g19v;
         }
+        if (L.g7.cf) {  // is the stencil form the matrix?
+            HM_CUDA(cudaStreamSynchronize(st));
+            g7_settle(L);
+        }
         HM_CHECK(stencil_galerkin(grid3[0], grid3[1], grid3[2], L, C.A, g19v, st, schur));
         HM_PHASE("  P^T A P (stencil)", st);
         return HMFEM_OK;
@@ -859,21 +906,52 @@ int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *dwork,
             return HMFEM_OK;
         }
     }
-    Csr AP;
-    UnionArgs a0{};
-    a0.nrows = n;
-    a0.orow = L.A.rowptr; a0.ocol = L.A.col; a0.oval = L.A.val; a0.w = L.pw;
-    a0.irow = L.P.rowptr; a0.icol = L.P.col; a0.ival = nullptr;
-    HM_CHECK(run_union<0>(a0, AP, dwork, st));
-    HM_PHASE("  A P", st);
+    // ---- the general product: A P in padded rows, then P^T (A P)
+    if (!cptr0) {  // a 19-offset level that turned out not to be one
+        cptr0 = (long long *)dalloc(sizeof(long long) * ((long)n + 1));
+        if (!cptr0) return HMFEM_E_CUDA;
+        a0.irow = L.P.rowptr;
+        HM_CHECK(union_count<0>(a0, cptr0, st));
+        HM_CUDA(cudaStreamSynchronize(st));
+    }
+    int *len0 = (int *)dalloc(sizeof(int) * (n > 0 ? n : 1));
+    long long *cptr1 = (long long *)dalloc(sizeof(long long) * (nc + 1));
+    C.A.n = L.nc;
+    C.A.rowptr = (int *)dalloc(sizeof(int) * (nc + 1));
+    if (!len0 || !cptr1 || !C.A.rowptr) {
+        set_last_error("out of device memory (RAP)", __FILE__, __LINE__);
+        return HMFEM_E_CUDA;
+    }
+    a0.w = L.pw;
+    a0.irow = L.P.rowptr; a0.icol = L.P.col;
+    a0.cptr = cptr0;
+    a0.ucnt = len0;
+    HM_CHECK(union_rows<0>(a0, PIN_ERR, dwork, st));
     UnionArgs a1{};
     a1.nrows = L.nc;
-    a1.orow = L.R.rowptr; a1.ocol = L.R.col; a1.oval = nullptr; a1.w = L.pw;
-    a1.irow = AP.rowptr; a1.icol = AP.col; a1.ival = AP.val;
-    HM_CHECK(run_union<1>(a1, C.A, dwork, st));
-    HM_PHASE("  P^T (A P)", st);
+    a1.orow = L.R.rowptr; a1.ocol = L.R.col; a1.w = L.pw;
+    a1.icol = a0.pcol; a1.ival = a0.pval; a1.iptr = cptr0; a1.ilen = len0;
+    HM_CHECK(union_count<1>(a1, cptr1, st));
     HM_CUDA(cudaStreamSynchronize(st));
-    dfree(AP.rowptr); dfree(AP.col); dfree(AP.val);
+    HM_PHASE("  A P", st);
+    HM_CHECK(union_error(PIN_ERR));
+    a1.cptr = cptr1;
+    a1.ucnt = C.A.rowptr;
+    HM_CHECK(union_rows<1>(a1, PIN_ERR2, dwork, st));
+    HM_CHECK(rowptr_from_counts(C.A.rowptr, L.nc, st, &C.A.nnz));  // synchronises
+    HM_CHECK(union_error(PIN_ERR2));
+    C.A.col = (int *)dalloc(sizeof(int) * (C.A.nnz > 0 ? C.A.nnz : 1));
+    C.A.val = (double *)dalloc(sizeof(double) * (C.A.nnz > 0 ? C.A.nnz : 1));
+    if (!C.A.col || !C.A.val) {
+        set_last_error("out of device memory (RAP)", __FILE__, __LINE__);
+        return HMFEM_E_CUDA;
+    }
+    k_compact<<<nblk(nc * 32, 256, 148L * 32), 256, 0, st>>>(cptr1, C.A.rowptr, L.nc, a1.pcol,
+                                                             a1.pval, C.A.col, C.A.val);
+    HM_LAUNCHED();
+    HM_PHASE("  P^T (A P)", st);
+    dfree(a0.pcol); dfree(a0.pval); dfree(a1.pcol); dfree(a1.pval);
+    dfree(cptr0); dfree(cptr1); dfree(len0);
     return HMFEM_OK;
 }
 

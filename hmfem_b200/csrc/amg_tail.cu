@@ -18,6 +18,8 @@
 // steps, 2.1 -> 0.26 ms; 482 -> 1, five steps, 2.2 -> 0.40 ms.  Above 512 rows
 // the bit sets no longer fit, and one SM would soon take longer than the
 // general path's launches.
+#include <string.h>
+
 #include "hm.cuh"
 
 namespace hm {
@@ -336,9 +338,11 @@ int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, Tail
         L0.A.n, L0.A.rowptr, L0.A.col, L0.A.val, l, max_levels, min_coarse, T.mem,
         (unsigned)kTailArena, ap, out);
     HM_LAUNCHED();
-    TailOut h;
-    HM_CUDA(cudaMemcpyAsync(&h, out, sizeof(TailOut), cudaMemcpyDeviceToHost, st));
+    static_assert(sizeof(TailOut) <= sizeof(int) * (PIN_WORDS - PIN_BLOCK), "pinned words");
+    HM_CHECK(read_back(PIN_BLOCK, out, (int)(sizeof(TailOut) / sizeof(int)), st));
     HM_CUDA(cudaStreamSynchronize(st));
+    TailOut h;
+    memcpy(&h, pinned_words() + PIN_BLOCK, sizeof(h));
     dfree(ap);
     dfree(out);
     for (int k = 0; k < h.levels; k++) {

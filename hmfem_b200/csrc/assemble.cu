@@ -79,15 +79,16 @@ __device__ __forceinline__ Faces cell_faces(const Grid &g, int i, int j, int k,
 
 struct FacePtrs { const double *l, *r, *u, *d, *t, *b; };
 
-__global__ void k_l0_rowcounts(int nx, int ny, int nz, int *cnt)
+// Entries of the rows before row s = (i, j, k): seven each, less the
+// neighbours missing at the faces.  (Counts, a scan and two read-backs of its
+// total took 60 to 160 us for what six comparisons give.)
+__device__ __forceinline__ long row_start(const Grid &g, long s, int i, int j, int k)
 {
-    long n = (long)nx * ny * nz;
-    for (long s = blockIdx.x * (long)blockDim.x + threadIdx.x; s < n;
-         s += (long)gridDim.x * blockDim.x) {
-        int i = (int)(s % nx), j = (int)((s / nx) % ny), k = (int)(s / ((long)nx * ny));
-        cnt[s] = 1 + (j > 0) + (i > 0) + (i < nx - 1) + (j < ny - 1) +
-                 (k < nz - 1) + (k > 0);
-    }
+    const long nx = g.nx, nxy = nx * g.ny, line = (long)k * g.ny + j;
+    const long x0 = line + (i > 0), x1 = line;
+    const long y0 = k * nx + (j > 0 ? nx : i), y1 = k * nx + (j == g.ny - 1 ? i : 0);
+    const long z0 = k > 0 ? nxy : s, z1 = k == g.nz - 1 ? s - k * nxy : 0;
+    return 7 * s - (x0 + x1 + y0 + y1 + z0 + z1);
 }
 
 // Right-hand side of cell s (source_term, set_source_term.c:23-220; faces in
@@ -140,7 +141,7 @@ k_assemble(Grid g, const double *__restrict__ KX, const double *__restrict__ KY,
            const double *__restrict__ KZ, FacePtrs fv,
            const double *__restrict__ KI, const double *__restrict__ WI,
            const double *__restrict__ PC, const double *__restrict__ PW,
-           const int *__restrict__ rowptr, int *__restrict__ col,
+           int *__restrict__ rowptr, int *__restrict__ col,
            double *__restrict__ val, double *__restrict__ b, int *bad)
 {
     const long nx = g.nx, nxy = (long)g.nx * g.ny, n = nxy * g.nz;
@@ -162,7 +163,8 @@ k_assemble(Grid g, const double *__restrict__ KX, const double *__restrict__ KY,
         // permeabilities.c:486: l + r + u + d + t + b + KI/(mu V) + WI/(mu V)
         double c = dadd(dadd(dadd(dadd(dadd(F.l, F.r), F.u), F.d), F.t), F.b);
         c = dadd(dadd(c, ki / g.kdiv), wi / g.kdiv);
-        long q = rowptr[s];
+        long q = row_start(g, s, i, j, k);
+        rowptr[s] = (int)q;
         if (j > 0)          { col[q] = (int)(s - nx);  val[q] = -F.d; q++; }
         if (i > 0)          { col[q] = (int)(s - 1);   val[q] = -F.l; q++; }
         col[q] = (int)s; val[q] = c; q++;
@@ -170,6 +172,7 @@ k_assemble(Grid g, const double *__restrict__ KX, const double *__restrict__ KY,
         if (j < g.ny - 1)   { col[q] = (int)(s + nx);  val[q] = -F.u; q++; }
         if (k < g.nz - 1)   { col[q] = (int)(s + nxy); val[q] = -F.t; q++; }
         if (k > 0)          { col[q] = (int)(s - nxy); val[q] = -F.b; q++; }
+        if (s == n - 1) rowptr[n] = (int)q;
         b[s] = cell_rhs(g, fv, i, j, k, s, F, ki, wi, PC ? PC[s] : 0.0, PW ? PW[s] : 0.0);
     }
 }
@@ -292,19 +295,11 @@ int grid_for(long n, int threads)
 
 }  // namespace
 
-int launch_l0_rowcounts(int nx, int ny, int nz, int *cnt, cudaStream_t st)
-{
-    long n = (long)nx * ny * nz;
-    k_l0_rowcounts<<<grid_for(n, 256), 256, 0, st>>>(nx, ny, nz, cnt);
-    HM_LAUNCHED();
-    return HMFEM_OK;
-}
-
 int launch_assemble(int nx, int ny, int nz, double hx, double hy, double hz,
                     double visc, const double *KX, const double *KY,
                     const double *KZ, const int bc[6], double *const face[6],
                     const double *KI, const double *WI, const double *pc,
-                    const double *pw, const int *rowptr, int *col, double *val,
+                    const double *pw, int *rowptr, int *col, double *val,
                     double *b, cudaStream_t st, int *bad)
 {
     Grid g = make_grid(nx, ny, nz, hx, hy, hz, visc, bc);

@@ -1254,6 +1254,9 @@ __global__ void k_fill_one(double *x, int n)
 // reported 0); the difference between levels l and l+1 is level l's share.
 int time_kernel(Solver &s, int which, int l, int reps, float *ms, double *bytes)
 {
+    // (levels below the coarse solve have no solve-phase forms until now)
+    if (s.direct_level >= 0 && l >= s.direct_level && l < s.nlevels)
+        HM_CHECK(level_forms(s, s.direct_level, s.nlevels - 1, -1, s.st));
     if (which == 12) {
         if (l < 0 || l >= s.nlevels || reps < 1) return HMFEM_E_ARG;
         cudaStream_t st = s.st;

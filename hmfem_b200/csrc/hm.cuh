@@ -134,12 +134,11 @@ enum { RED_TAU = 0, RED_RR, RED_SIGMA, RED_TRR, RED_BB, RED_A, RED_B, RED_C,
 
 // ---- launchers (all enqueue on `st`) ---------------------------------
 // assembly / flux (assemble.cu)
-int launch_l0_rowcounts(int nx, int ny, int nz, int *cnt, cudaStream_t st);
 int launch_assemble(int nx, int ny, int nz, double hx, double hy, double hz,
                     double visc, const double *KX, const double *KY,
                     const double *KZ, const int bc[6], double *const face[6],
                     const double *KI, const double *WI, const double *pc,
-                    const double *pw, const int *rowptr, int *col, double *val,
+                    const double *pw, int *rowptr, int *col, double *val,
                     double *b, cudaStream_t st, int *bad = nullptr);
 int launch_exchange_rhs(int nx, int ny, int nz, double hx, double hy, double hz,
                         double visc, const double *KX, const double *KY,
@@ -156,10 +155,32 @@ int launch_flux(int nx, int ny, int nz, double hx, double hy, double hz,
                 const double *p, hmfem_ele *v, double *mm, cudaStream_t st);
 
 // sparse utilities (sparse.cu)
+// Sizes and flags the host needs: copied into pinned words of the solver
+// (read_back, by slot) as they are produced and looked at after one
+// synchronisation for several of them.
+enum PinSlot {
+    PIN_TOTAL = 0, PIN_ERR, PIN_ERR2, PIN_NC, PIN_P, PIN_R, PIN_RBAD, PIN_NNZ, PIN_G7, PIN_DENSE,
+    PIN_DIAG, PIN_CAND = 12 /* 2 words */, PIN_SELL = 14 /* 2 words */, PIN_PACK = 16,
+    PIN_LEVELS = 64 /* 2 words per level */, PIN_FLAGS = 192 /* 1 word per level */,
+    PIN_BLOCK = 256, PIN_WORDS = 4096
+};
+int *pinned_words();
+int read_back(int slot, const void *src, int words, cudaStream_t st);
 int scan_exclusive(const int *in, int *out, int n, cudaStream_t st);
+// counts to row pointers (n + 1 entries) without a read-back; the total once
+// it has been read back into a slot and waited for; both at once
+int rowptr_scan(int *rowptr, int n, cudaStream_t st);
+int rowptr_total(int slot, long *nnz_out);
 int rowptr_from_counts(int *rowptr, int n, cudaStream_t st, long *nnz_out);
 int csr_to_sell(const Csr &A, Sell &S, cudaStream_t st);
 int sell_fill_lowp(Sell &S, bool f32, bool bf16, cudaStream_t st);
+// the same in halves, for many levels between two synchronisations: slices
+// and their total length (read back into slot, 2 words), the entries; the
+// reduced-precision values (*bad set where sell_unpack has to follow)
+int sell_layout(const Csr &A, Sell &S, int slot, cudaStream_t st);
+int sell_fill(const Csr &A, Sell &S, int slot, cudaStream_t st);
+int sell_lowp(Sell &S, bool f32, bool bf16, int *bad, cudaStream_t st);
+void sell_unpack(Sell &S);
 struct Level;
 int csr_fill_lowp(Level &L, bool bf16, cudaStream_t st);
 int launch_diag_inv(const Csr &A, double *dinv, float *dinv32, cudaStream_t st,
@@ -189,6 +210,11 @@ int stencil_parity_split(int nx, int ny, int nz, signed char *sel, cudaStream_t 
 // R = P^T of the parity split (rowptr / col allocated by the caller, R.nnz
 // set to P's nnz)
 int stencil_parity_R(int nx, int ny, int nz, const int *cid, int nc, Csr &R, cudaStream_t st);
+// sizes of the parity split of a grid: C cells, entries of P (and of R), and
+// of the 19-offset Galerkin level
+long parity_coarse(int nx, int ny, int nz);
+long parity_pnnz(int nx, int ny, int nz);
+long parity_galerkin_nnz(int nx, int ny, int nz);
 // level 1 of a parity split (nx even, nx, ny >= 4): its greedy C/F split
 // from the 19-offset structure, the x-row wavefront in one launch; work
 // holds stencil19_split_work_ints(nx, ny, nz) ints (8-byte aligned), the
@@ -205,18 +231,24 @@ int stencil_galerkin(int nx, int ny, int nz, const Level &L, Csr &out,
 // parity split) from that structure, bit-identical to the generic product;
 // *done false (and out untouched) when the level does not have it
 int galerkin19(const Level &L, Csr &out, cudaStream_t st, bool *done);
-// R = P^T of such a level from its structure (R.rowptr / R.col allocated by
-// the caller, P formed); *done false when the level does not have it
-int g19_transpose(const Level &L, Csr &R, cudaStream_t st, bool *done);
+// R = P^T of such a level from its structure: the row pointers (R.rowptr of
+// at least nc + 1 entries; the total is read back into PIN_R, a flag into
+// PIN_RBAD), then,
+// when those agree with P, the columns
+bool g19_has_structure(const Level &L);
+int g19_transpose_rows(const Level &L, Csr &R, int *bad, cudaStream_t st);
+int g19_transpose_fill(const Level &L, Csr &R, cudaStream_t st);
 // L.cpts of such a level (its C rows in coarse-id order, for galerkin19)
 int g19_cpts(Level &L, cudaStream_t st);
 // colouring + rows grouped by colour; returns HMFEM_OK with L.gs = false
 // when the level needs more than 63 colours
 int color_level(Level &L, cudaStream_t st, int *dwork);
 // structured solve-phase forms (stencil_cycle.cu): g7_build fills L.g7 from
-// the assembled CSR and returns HMFEM_OK with L.g7.c == nullptr when the
-// matrix is not bitwise symmetric; g19 values come from stencil_galerkin.
+// the assembled CSR; whether the matrix is bitwise symmetric is read back into
+// PIN_G7 and, once waited for, g7_settle drops the form if it is not; g19
+// values come from stencil_galerkin.
 int g7_build(Level &L, int nx, int ny, int nz, bool f32, cudaStream_t st, int *dwork);
+void g7_settle(Level &L);
 void g7_free(Grid7 &g);
 bool g19_applies(int nx, int ny, int nz);
 int g19_lowp(Grid19 &g, int n, bool f32, bool bf16, cudaStream_t st);
@@ -237,6 +269,9 @@ struct AllocCache;                       // per-solver exact-size block cache
 void set_alloc_context(cudaStream_t st, AllocCache *c);
 void get_alloc_context(cudaStream_t *st, AllocCache **c);
 AllocCache *alloc_cache_new();
+// kPinExtra pinned bytes of the cache's owner (null when there are none)
+constexpr size_t kPinExtra = 4096;
+void *pinned_extra(AllocCache *c);
 void alloc_cache_release(AllocCache *c);
 
 }  // namespace hm

@@ -498,32 +498,39 @@ int blocks_for(long n, int threads, long cap = 148L * 16)
 
 }  // namespace
 
-int g19_transpose(const Level &L, Csr &R, cudaStream_t st, bool *done)
+bool g19_has_structure(const Level &L)
 {
-    *done = false;
     const Grid19 &gg = L.g19;
-    if (gg.nx <= 0 || (gg.nx & 1) || gg.nx < 4 || gg.ny < 4) return HMFEM_OK;
-    if ((long)gg.nx * gg.ny * gg.nz > (1l << 30)) return HMFEM_OK;
-    const G19L g{gg.nx, gg.ny, gg.nz, gg.nx / 2, gg.nx * gg.ny};
+    return gg.nx > 0 && !(gg.nx & 1) && gg.nx >= 4 && gg.ny >= 4 &&
+           (long)gg.nx * gg.ny * gg.nz <= (1l << 30) &&
+           (long)L.A.n == (long)(gg.nx / 2) * gg.ny * gg.nz;
+}
+
+static G19L g19_grid(const Level &L)
+{
+    const Grid19 &gg = L.g19;
+    return G19L{gg.nx, gg.ny, gg.nz, gg.nx / 2, gg.nx * gg.ny};
+}
+
+int g19_transpose_rows(const Level &L, Csr &R, int *bad, cudaStream_t st)
+{
     const long n = L.A.n;
-    if (n != (long)g.hx * g.ny * g.nz || L.nc < 1) return HMFEM_OK;
-    int *bad = (int *)dalloc(sizeof(int));
-    if (!bad) return HMFEM_E_CUDA;
     HM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
     HM_CUDA(cudaMemsetAsync(R.rowptr, 0, sizeof(int) * ((long)L.nc + 1), st));
-    k_g19_rcount<<<blocks_for(n, 256), 256, 0, st>>>(g, (int)n, L.A.rowptr, L.sel, L.cid,
-                                                      R.rowptr, bad);
+    k_g19_rcount<<<blocks_for(n, 256), 256, 0, st>>>(g19_grid(L), (int)n, L.A.rowptr, L.sel,
+                                                     L.cid, R.rowptr, bad);
     HM_LAUNCHED();
-    int hbad = 0;
-    HM_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-    long nnz = 0;
-    HM_CHECK(rowptr_from_counts(R.rowptr, L.nc, st, &nnz));  // synchronises
-    dfree(bad);
-    // not this structure: the radix sort forms R
-    if (hbad || nnz != L.P.nnz) return HMFEM_OK;
-    k_g19_rfill<<<blocks_for(n, 256), 256, 0, st>>>(g, (int)n, L.sel, L.cid, R.rowptr, R.col);
+    HM_CHECK(rowptr_scan(R.rowptr, L.nc, st));
+    HM_CHECK(read_back(PIN_RBAD, bad, 1, st));
+    return read_back(PIN_R, R.rowptr + L.nc, 1, st);
+}
+
+int g19_transpose_fill(const Level &L, Csr &R, cudaStream_t st)
+{
+    const long n = L.A.n;
+    k_g19_rfill<<<blocks_for(n, 256), 256, 0, st>>>(g19_grid(L), (int)n, L.sel, L.cid, R.rowptr,
+                                                    R.col);
     HM_LAUNCHED();
-    *done = true;
     return HMFEM_OK;
 }
 
@@ -580,10 +587,9 @@ int galerkin19(const Level &L, Csr &out, cudaStream_t st, bool *done)
                                         out.rowptr, pcol, pval, err);
     HM_LAUNCHED();
     HM_PHASE("    coarse rows", st);
-    int herr = 0;
-    HM_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    HM_CHECK(read_back(PIN_ERR, err, 1, st));
     HM_CHECK(rowptr_from_counts(out.rowptr, (int)nc, st, &out.nnz));  // synchronises
-    if (herr) {  // not this structure after all: the generic product runs
+    if (pinned_words()[PIN_ERR]) {  // not this structure after all: the generic product runs
         release();
         dfree(out.rowptr);
         out = Csr();

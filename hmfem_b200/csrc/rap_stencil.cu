@@ -569,6 +569,42 @@ int stencil_parity_split(int nx, int ny, int nz, signed char *sel, cudaStream_t 
     return HMFEM_OK;
 }
 
+// cells of the a x b x c box with its corner at (x, y, z) whose coordinate
+// sum is even
+static long even_cells(long x, long y, long z, long a, long b, long c)
+{
+    if (a <= 0 || b <= 0 || c <= 0) return 0;
+    const long v = a * b * c;
+    return (v & 1) && ((x + y + z) & 1) ? v / 2 : (v + 1) / 2;
+}
+
+long parity_coarse(int nx, int ny, int nz) { return even_cells(0, 0, 0, nx, ny, nz); }
+
+// every C cell's own entry, and one for every grid edge (it joins a C cell
+// and an F cell that interpolates from it)
+long parity_pnnz(int nx, int ny, int nz)
+{
+    const long x = nx, y = ny, z = nz;
+    return parity_coarse(nx, ny, nz) + (x - 1) * y * z + x * (y - 1) * z + x * y * (z - 1);
+}
+
+// per offset, the even cells whose neighbour there is in the grid
+long parity_galerkin_nnz(int nx, int ny, int nz)
+{
+    long t = 0;
+    const int n[3] = {nx, ny, nz};
+    for (int q = 0; q < 19; q++) {
+        const int o[3] = {OX(q), OY(q), OZ(q)};
+        long lo[3], len[3];
+        for (int d = 0; d < 3; d++) {
+            lo[d] = o[d] < 0 ? -o[d] : 0;
+            len[d] = n[d] - (o[d] < 0 ? -o[d] : o[d]);
+        }
+        t += even_cells(lo[0], lo[1], lo[2], len[0], len[1], len[2]);
+    }
+    return t;
+}
+
 int stencil_galerkin(int nx, int ny, int nz, const Level &L, Csr &out,
                      double *g19v, cudaStream_t st, bool schur)
 {
@@ -579,7 +615,12 @@ int stencil_galerkin(int nx, int ny, int nz, const Level &L, Csr &out,
     if (!out.rowptr) return HMFEM_E_CUDA;
     k_sg_count<<<nbk(n / 2), 256, 0, st>>>(g, L.cid, out.rowptr);
     HM_LAUNCHED();
-    HM_CHECK(rowptr_from_counts(out.rowptr, L.nc, st, &out.nnz));
+    HM_CHECK(rowptr_scan(out.rowptr, L.nc, st));
+    out.nnz = parity_galerkin_nnz(nx, ny, nz);
+    if (out.nnz > 2147483647L) {
+        set_last_error("more than 2^31-1 nonzeros", __FILE__, __LINE__);
+        return HMFEM_E_CAPACITY;
+    }
     out.col = (int *)dalloc(sizeof(int) * (out.nnz > 0 ? out.nnz : 1));
     out.val = (double *)dalloc(sizeof(double) * (out.nnz > 0 ? out.nnz : 1));
     if (!out.col || !out.val) return HMFEM_E_CUDA;
@@ -612,12 +653,7 @@ int stencil_parity_R(int nx, int ny, int nz, const int *cid, int nc, Csr &R, cud
     HM_CUDA(cudaMemsetAsync(R.rowptr, 0, sizeof(int) * ((long)nc + 1), st));
     k_parity_rcount<<<nbk(n / 2), 256, 0, st>>>(g, cid, R.rowptr);
     HM_LAUNCHED();
-    long nnz = 0;
-    HM_CHECK(rowptr_from_counts(R.rowptr, nc, st, &nnz));
-    if (nnz != R.nnz) {
-        set_last_error("parity split: R size differs from P", __FILE__, __LINE__);
-        return HMFEM_E_CAPACITY;
-    }
+    HM_CHECK(rowptr_scan(R.rowptr, nc, st));
     k_parity_rfill<<<nbk(n / 2), 256, 0, st>>>(g, cid, R.rowptr, R.col);
     HM_LAUNCHED();
     return HMFEM_OK;

@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 
 #include "cycle.cuh"
 
@@ -540,8 +541,10 @@ int small_cycle_build(Solver &s, cudaStream_t st)
         k_sc_scan<<<dim3(q.levels, ctas + 1), 256, 0, st>>>(q, dev, S.masks);
         HM_LAUNCHED();
         ScFound h[kScLevels][kScCtas + 1];
-        HM_CUDA(cudaMemcpyAsync(h, dev, sizeof(h), cudaMemcpyDeviceToHost, st));
+        static_assert(sizeof(h) <= sizeof(int) * (PIN_WORDS - PIN_BLOCK), "pinned words");
+        HM_CHECK(read_back(PIN_BLOCK, dev, (int)(sizeof(h) / sizeof(int)), st));
         HM_CUDA(cudaStreamSynchronize(st));
+        memcpy(h, pinned_words() + PIN_BLOCK, sizeof(h));
         auto most = [&](int l, int k) {
             int m = 0;
             for (int c = 0; c < ctas; c++) m = std::max(m, h[l - lo][c + 1].at[k] - h[l - lo][c].at[k]);

@@ -192,11 +192,19 @@ int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st)
     return HMFEM_OK;
 }
 
-__global__ void k_fill(double *p, long n, double v)
+// constant values of the boundary faces (n = 0: given by the caller)
+struct FaceFill {
+    double *p[6];
+    long n[6];
+    double v[6];
+};
+
+__global__ void k_fill_faces(FaceFill a)
 {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+    const int f = blockIdx.y;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.n[f];
          i += (long)gridDim.x * blockDim.x)
-        p[i] = v;
+        a.p[f][i] = a.v[f];
 }
 
 // ---- helpers -------------------------------------------------------------
@@ -246,11 +254,11 @@ static void free_level_setup(Level &L, bool keep_matrix)
     if (keep_matrix) L.A = a;
 }
 
+// The captured iteration is stale; its executable graph is kept, to be updated
+// by the next capture (a hierarchy of the same levels has the same graph).
 static void drop_graph(Solver &s)
 {
-    if (s.gexec) cudaGraphExecDestroy(s.gexec);
     if (s.graph) cudaGraphDestroy(s.graph);
-    s.gexec = nullptr;
     s.graph = nullptr;
 }
 
@@ -391,6 +399,61 @@ static int alloc_level_vectors(Solver &s, Level &L)
     return HMFEM_OK;
 }
 
+// Solve-phase forms of levels k0 .. k1 that lack them: SELL-32 where no
+// structured form applies, the smoother's diagonal, the cycle's vectors;
+// level `dense` is solved by its inverse and needs only vectors.  Two
+// synchronisations for all of them (the slices' lengths, whether the packed
+// form holds every column).
+int level_forms(Solver &s, int k0, int k1, int dense, cudaStream_t st)
+{
+    const bool low = s.opt.precision == 1;
+    std::vector<int> todo, check;
+    for (int k = k0; k <= k1; k++) {
+        Level &L = s.lv[k];
+        // (level 0 is also the CG's matrix)
+        if ((k != dense || k == 0) && !s.use_g7(k) && !s.use_g19(k) && !L.S.sptr) {
+            todo.push_back(k);
+            HM_CHECK(sell_layout(L.A, L.S, PIN_LEVELS + 2 * k, st));
+        }
+        if (k != dense && !L.dsm) {
+            HM_ALLOC(L.dsm, double, L.A.n);
+            HM_ALLOC(L.dsm32, float, L.A.n);
+            // Chebyshev levels always use the l1 diagonal (its bound 1 on the
+            // spectrum of D^-1 A fixes the Chebyshev interval)
+            HM_CHECK(launch_smoother_diag(L.A, L.cheb ? 1 : s.opt.smoother, L.dsm, L.dsm32, st));
+        }
+        if (!L.f) HM_CHECK(alloc_level_vectors(s, L));
+        if (L.cheb && !L.dx) {
+            HM_ALLOC(L.dx, double, L.A.n);
+            if (low) HM_ALLOC(L.dx32, float, L.A.n);
+        }
+    }
+    HM_CUDA(cudaStreamSynchronize(st));
+    int *flags = s.dwork + 16;  // by level
+    HM_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * 48, st));
+    for (int k : todo) {
+        Level &L = s.lv[k];
+        HM_CHECK(sell_fill(L.A, L.S, PIN_LEVELS + 2 * k, st));
+        if (!low) continue;
+        if (k >= 48) {
+            HM_CHECK(sell_fill_lowp(L.S, true, s.use_bf16(k), st));
+            continue;
+        }
+        HM_CHECK(sell_lowp(L.S, true, s.use_bf16(k), flags + k, st));
+        // up to 32768 rows every column is within the packed form's reach
+        if (L.S.pk && L.A.n > 32768) {
+            check.push_back(k);
+            HM_CHECK(read_back(PIN_FLAGS + k, flags + k, 1, st));
+        }
+    }
+    if (!check.empty()) {
+        HM_CUDA(cudaStreamSynchronize(st));
+        for (int k : check)
+            if (pinned_words()[PIN_FLAGS + k]) sell_unpack(s.lv[k].S);
+    }
+    return HMFEM_OK;
+}
+
 int setup(Solver &s)
 {
     if (s.lv.empty() || !s.lv[0].A.col) {
@@ -454,6 +517,10 @@ int setup(Solver &s)
         rel = (double)gcnt / (double)gold;
     }
     s.nlevels = l + 1;
+    if (l == 0 && s.lv[0].g7.cf) {  // not coarsened: is the stencil form the matrix?
+        HM_CUDA(cudaStreamSynchronize(st));
+        g7_settle(s.lv[0]);
+    }
     HM_PHASE("setup: hierarchy", st);
     if (s.schur0_built && !s.use_g7(0)) {
         // the reduction needs the stencil form of level 0 (a bitwise
@@ -472,48 +539,33 @@ int setup(Solver &s)
         else
             g19_free(s.lv[1].g19);
     }
-    // solve-phase formats and vectors
-    for (int k = 0; k < s.nlevels; k++) {
-        Level &L = s.lv[k];
-        if (!s.use_g7(k) && !s.use_g19(k)) {
-            HM_CHECK(csr_to_sell(L.A, L.S, st));
-            if (low) HM_CHECK(sell_fill_lowp(L.S, true, s.use_bf16(k), st));
-        }
-        HM_ALLOC(L.dsm, double, L.A.n);
-        HM_ALLOC(L.dsm32, float, L.A.n);
-        // Chebyshev levels always use the l1 diagonal (its bound 1 on the
-        // spectrum of D^-1 A fixes the Chebyshev interval)
-        HM_CHECK(launch_smoother_diag(L.A, L.cheb ? 1 : s.opt.smoother, L.dsm, L.dsm32, st));
-        HM_CHECK(alloc_level_vectors(s, L));
-        if (L.cheb) {
-            HM_ALLOC(L.dx, double, L.A.n);
-            if (low) HM_ALLOC(L.dx32, float, L.A.n);
-        }
-    }
-    HM_PHASE("setup: SELL + vectors", st);
     // dense coarse solve on the first level small enough
     s.direct_level = -1;
+    int dense = -1;
     if (s.opt.coarse_direct > 0) {
-        for (int k = 0; k < s.nlevels; k++) {
-            if (s.lv[k].A.n <= s.opt.coarse_direct && s.lv[k].A.n <= kDenseMax) {
-                const long n = s.lv[k].A.n;
-                HM_ALLOC(s.dense_L, double, n * n);
-                HM_CUDA(cudaMemsetAsync(s.dwork, 0, sizeof(int), st));
-                HM_CHECK(dense_factor(s.lv[k].A, s.dense_L, s.dwork, st));
-                int err = 0;
-                HM_CUDA(cudaMemcpyAsync(&err, s.dwork, sizeof(int), cudaMemcpyDeviceToHost, st));
-                HM_CUDA(cudaStreamSynchronize(st));
-                if (err) {  // not SPD: keep the reference's diagonal solve
-                    dfree(s.dense_L);
-                    s.dense_L = nullptr;
-                } else {
-                    s.direct_level = k;
-                }
-                HM_PHASE("setup: coarse inverse", st);
-                break;
-            }
+        for (int k = 0; k < s.nlevels && dense < 0; k++)
+            if (s.lv[k].A.n <= s.opt.coarse_direct && s.lv[k].A.n <= kDenseMax) dense = k;
+        if (dense >= 0) {
+            const long n = s.lv[dense].A.n;
+            HM_ALLOC(s.dense_L, double, n * n);
+            HM_CUDA(cudaMemsetAsync(s.dwork, 0, sizeof(int), st));
+            HM_CHECK(dense_factor(s.lv[dense].A, s.dense_L, s.dwork, st));
+            HM_CHECK(read_back(PIN_DENSE, s.dwork, 1, st));
         }
     }
+    // solve-phase formats and vectors of the levels the cycle visits (those
+    // below the coarse solve get theirs when something asks for them)
+    HM_CHECK(level_forms(s, 0, dense >= 0 ? dense : s.nlevels - 1, dense, st));
+    if (dense >= 0) {
+        if (pinned_words()[PIN_DENSE]) {  // not SPD: keep the reference's diagonal solve
+            dfree(s.dense_L);
+            s.dense_L = nullptr;
+            HM_CHECK(level_forms(s, dense, s.nlevels - 1, -1, st));
+        } else {
+            s.direct_level = dense;
+        }
+    }
+    HM_PHASE("setup: formats, coarse inverse", st);
     // multicolour Gauss-Seidel on the coarse levels above the coarse solve
     if (s.opt.gs_from >= 1) {
         const int stop = s.direct_level >= 0 ? s.direct_level : s.nlevels - 1;
@@ -525,10 +577,10 @@ int setup(Solver &s)
         }
         HM_PHASE("setup: colouring", st);
     }
+    HM_CHECK(read_back(PIN_DIAG, s.dwork + 8, 1, st));
     HM_CHECK(small_cycle_build(s, st));
-    int nonpos = 0;
-    HM_CUDA(cudaMemcpyAsync(&nonpos, s.dwork + 8, sizeof(int), cudaMemcpyDeviceToHost, st));
     HM_CUDA(cudaStreamSynchronize(st));
+    const int nonpos = pinned_words()[PIN_DIAG];
     if (nonpos) {
         char msg[160];
         snprintf(msg, sizeof(msg),
@@ -560,6 +612,13 @@ static int capture_iteration(Solver &s)
     }
     HM_CUDA(e);
     s.graph = g;
+    if (s.gexec) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(s.gexec, g, &info) == cudaSuccess) return HMFEM_OK;
+        cudaGetLastError();  // another graph: instantiate it
+        cudaGraphExecDestroy(s.gexec);
+        s.gexec = nullptr;
+    }
     HM_CUDA(cudaGraphInstantiate(&s.gexec, g, 0));
     return HMFEM_OK;
 }
@@ -596,7 +655,7 @@ int solve(Solver &s, const double *b, double *x, int mem, hmfem_stats *out)
     HM_PHASE(nullptr, st);
     int rc = cg_init(s, st);
     HM_PHASE("solve: init", st);
-    if (rc == HMFEM_OK && !s.gexec) rc = capture_iteration(s);
+    if (rc == HMFEM_OK && !s.graph) rc = capture_iteration(s);
     s.ctl_active = false;
     if (rc != HMFEM_OK) return rc;
     // chunks of k iterations, one chunk kept queued ahead of the host check
@@ -931,8 +990,9 @@ int hmfem_create(hmfem_solver **out, const hmfem_options *opt)
     s.dwork = (int *)hm::dalloc(sizeof(int) * 64);
     s.mm = (double *)hm::dalloc(sizeof(double) * 2);
     s.gsbar = (unsigned *)hm::dalloc(sizeof(unsigned) * 4);
-    if (cudaMallocHost(&s.ctl_host, 2 * sizeof(hm::Ctl)) != cudaSuccess ||
-        !s.ctl || !s.part || !s.dwork || !s.mm || !s.gsbar) {
+    static_assert(2 * sizeof(hm::Ctl) <= hm::kPinExtra, "pinned control blocks");
+    s.ctl_host = (hm::Ctl *)hm::pinned_extra(s.cache);
+    if (!s.ctl_host || !s.ctl || !s.part || !s.dwork || !s.mm || !s.gsbar) {
         hm::set_last_error("out of memory", __FILE__, __LINE__);
         hmfem_destroy(h);
         return HMFEM_E_CUDA;
@@ -952,6 +1012,7 @@ int hmfem_destroy(hmfem_solver *h)
     if (s.st) cudaStreamSynchronize(s.st);
     hm::karst_release(s);
     hm::free_hierarchy(s, false);
+    if (s.gexec) cudaGraphExecDestroy(s.gexec);
     hm::free_vectors(s);
     for (int i = 0; i < 3; i++) hm::dfree(s.Kown[i]);
     for (int f = 0; f < 6; f++) hm::dfree(s.face[f]);
@@ -962,7 +1023,6 @@ int hmfem_destroy(hmfem_solver *h)
     hm::alloc_cache_release(s.cache);
     s.cache = nullptr;
     hm::set_alloc_context(s.st, nullptr);
-    if (s.ctl_host) cudaFreeHost(s.ctl_host);
     if (s.st) cudaStreamSynchronize(s.st);
     if (s.own_stream && s.st) cudaStreamDestroy(s.st);
     // the thread's allocation context must not keep naming a dead stream
@@ -1058,32 +1118,38 @@ int hmfem_assemble(hmfem_solver *h, int nx, int ny, int nz, double hx,
     // face values in the Bound layout (l,r: ny*nz; u,d: nx*nz; t,b: nx*ny)
     const long fsz[6] = {(long)ny * nz, (long)ny * nz, (long)nx * nz,
                          (long)nx * nz, (long)nx * ny, (long)nx * ny};
+    hm::FaceFill fill{};
+    long most = 0;
     for (int f = 0; f < 6; f++) {
         if (!s.face[f]) HM_ALLOC(s.face[f], double, fsz[f]);
         if (face_vals && face_vals[f]) {
             HM_CHECK(hm::upload(s.face[f], face_vals[f], fsz[f], mem, st));
         } else {
-            double v = bc_value ? bc_value[f] : 0.0;
-            hm::k_fill<<<(int)hm::ceil_div(fsz[f], 256) < 1024 ? (int)hm::ceil_div(fsz[f], 256) : 1024,
-                         256, 0, st>>>(s.face[f], fsz[f], v);
-            HM_LAUNCHED();
+            fill.p[f] = s.face[f];
+            fill.n[f] = fsz[f];
+            fill.v[f] = bc_value ? bc_value[f] : 0.0;
+            most = most > fsz[f] ? most : fsz[f];
         }
+    }
+    if (most > 0) {
+        hm::k_fill_faces<<<dim3((unsigned)std::min(hm::ceil_div(most, 256), (int64_t)512), 6), 256, 0,
+                           st>>>(fill);
+        HM_LAUNCHED();
     }
     hm::Level &L = s.lv[0];
     HM_PHASE("assemble: buffers + faces", st);
-    HM_CHECK(hm::launch_l0_rowcounts(nx, ny, nz, L.A.rowptr, st));
-    HM_CHECK(hm::rowptr_from_counts(L.A.rowptr, (int)n, st, &L.A.nnz));
+    // one entry per cell and two per interior face
+    L.A.nnz = 7 * n - 2 * (fsz[0] + fsz[2] + fsz[4]);
     HM_ALLOC(L.A.col, int, L.A.nnz);
     HM_ALLOC(L.A.val, double, L.A.nnz);
-    HM_PHASE("assemble: row pointers", st);
     HM_CUDA(cudaMemsetAsync(s.dwork, 0, sizeof(int), st));
     HM_CHECK(hm::launch_assemble(nx, ny, nz, hx, hy, hz, visc, s.KX, s.KY, s.KZ,
                                  s.bc, s.face, nullptr, nullptr, nullptr,
                                  nullptr, L.A.rowptr, L.A.col, L.A.val, s.b, st,
                                  s.dwork));
-    int bad = 0;
-    HM_CUDA(cudaMemcpyAsync(&bad, s.dwork, sizeof(int), cudaMemcpyDeviceToHost, st));
+    HM_CHECK(hm::read_back(hm::PIN_ERR, s.dwork, 1, st));
     HM_CUDA(cudaStreamSynchronize(st));
+    const int bad = hm::pinned_words()[hm::PIN_ERR];
     HM_PHASE("assemble: TPFA kernel", st);
     s.setup_done = false;
     s.bad_matrix = bad != 0;

@@ -171,6 +171,7 @@ int g19_spmv(const Level &L, const double *x, double *y, cudaStream_t st);
 
 // solver.cu entry points the coupled driver (karst.cu) builds on
 int setup(Solver &s);
+int level_forms(Solver &s, int k0, int k1, int dense, cudaStream_t st);
 int solve(Solver &s, const double *b, double *x, int mem, hmfem_stats *out);
 int profile_iteration(Solver &s, int iters, hmfem_kernel_time *out, int cap, int *count);
 int batch_solve(Solver *const *ss, int m, double *const *x, int mem, hmfem_stats *out);

@@ -1,6 +1,7 @@
 // sparse.cu -- scans, CSR -> SELL-32 conversion, diagonal extraction and the
 // FP64 SELL SpMV.
 #include <cstdlib>
+#include <cstring>
 #include <cub/device/device_scan.cuh>
 #include <atomic>
 #include <map>
@@ -49,9 +50,11 @@ static std::atomic<unsigned> g_pool_ready{0};  // bit per device
 
 // Per-solver cache of freed blocks keyed by exact size: a solver that sets
 // up the same grid again gets every buffer back without touching the pool.
+// It also carries the pinned words that size and flag read-backs land in.
 struct AllocCache {
     std::unordered_map<void *, size_t> live;
     std::multimap<size_t, void *> idle;
+    int *pinned = nullptr;
 };
 static thread_local AllocCache *g_cache = nullptr;
 
@@ -69,7 +72,30 @@ void get_alloc_context(cudaStream_t *st, AllocCache **c)
     *c = g_cache;
 }
 
-AllocCache *alloc_cache_new() { return new AllocCache(); }
+AllocCache *alloc_cache_new()
+{
+    AllocCache *c = new AllocCache();
+    if (cudaMallocHost(&c->pinned, sizeof(int) * PIN_WORDS + kPinExtra) != cudaSuccess) {
+        cudaGetLastError();
+        c->pinned = nullptr;
+    }
+    return c;
+}
+
+int *pinned_words()
+{
+    static thread_local int words[PIN_WORDS];
+    return g_cache && g_cache->pinned ? g_cache->pinned : words;
+}
+
+void *pinned_extra(AllocCache *c) { return c->pinned ? c->pinned + PIN_WORDS : nullptr; }
+
+int read_back(int slot, const void *src, int words, cudaStream_t st)
+{
+    HM_CUDA(cudaMemcpyAsync(pinned_words() + slot, src, sizeof(int) * words,
+                            cudaMemcpyDeviceToHost, st));
+    return HMFEM_OK;
+}
 
 void alloc_cache_release(AllocCache *c)
 {
@@ -77,6 +103,10 @@ void alloc_cache_release(AllocCache *c)
     for (auto &kv : c->idle) cudaFreeAsync(kv.second, g_astream);
     for (auto &kv : c->live) cudaFreeAsync(kv.first, g_astream);
     if (g_cache == c) g_cache = nullptr;
+    if (c->pinned) {
+        cudaStreamSynchronize(g_astream);
+        cudaFreeHost(c->pinned);
+    }
     delete c;
 }
 
@@ -172,9 +202,25 @@ int scan_exclusive(const int *in, int *out, int n, cudaStream_t st)
     void *t = dalloc(tmp);
     if (!t) { set_last_error("out of device memory (scan)", __FILE__, __LINE__); return HMFEM_E_CUDA; }
     cudaError_t e = cub::DeviceScan::ExclusiveSum(t, tmp, in, out, n, st);
-    cudaStreamSynchronize(st);
-    dfree(t);
+    dfree(t);  // reused, if at all, by later work of the same stream
     HM_CUDA(e);
+    return HMFEM_OK;
+}
+
+int rowptr_scan(int *rowptr, int n, cudaStream_t st)
+{
+    HM_CUDA(cudaMemsetAsync(rowptr + n, 0, sizeof(int), st));
+    return scan_exclusive(rowptr, rowptr, n + 1, st);
+}
+
+int rowptr_total(int slot, long *nnz_out)
+{
+    const int tot = pinned_words()[slot];
+    if (tot < 0) {  // the 32-bit sum wrapped
+        set_last_error("more than 2^31-1 nonzeros", __FILE__, __LINE__);
+        return HMFEM_E_CAPACITY;
+    }
+    *nnz_out = tot;
     return HMFEM_OK;
 }
 
@@ -182,27 +228,10 @@ int scan_exclusive(const int *in, int *out, int n, cudaStream_t st)
 // scan with rowptr[n] = total, which is returned in *nnz_out.
 int rowptr_from_counts(int *rowptr, int n, cudaStream_t st, long *nnz_out)
 {
-    int last = 0;
-    if (n > 0)
-        HM_CUDA(cudaMemcpyAsync(&last, rowptr + n - 1, sizeof(int),
-                                cudaMemcpyDeviceToHost, st));
-    HM_CHECK(scan_exclusive(rowptr, rowptr, n, st));
-    int base = 0;
-    if (n > 0)
-        HM_CUDA(cudaMemcpyAsync(&base, rowptr + n - 1, sizeof(int),
-                                cudaMemcpyDeviceToHost, st));
+    HM_CHECK(rowptr_scan(rowptr, n, st));
+    HM_CHECK(read_back(PIN_TOTAL, rowptr + n, 1, st));
     HM_CUDA(cudaStreamSynchronize(st));
-    long tot = (long)base + last;
-    if (tot > 2147483647L) {
-        set_last_error("more than 2^31-1 nonzeros", __FILE__, __LINE__);
-        return HMFEM_E_CAPACITY;
-    }
-    int t32 = (int)tot;
-    HM_CUDA(cudaMemcpyAsync(rowptr + n, &t32, sizeof(int),
-                            cudaMemcpyHostToDevice, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-    *nnz_out = tot;
-    return HMFEM_OK;
+    return rowptr_total(PIN_TOTAL, nnz_out);
 }
 
 namespace {
@@ -323,7 +352,7 @@ int nblocks(long n, int threads, long cap = 148L * 16)
 
 }  // namespace
 
-int csr_to_sell(const Csr &A, Sell &S, cudaStream_t st)
+int sell_layout(const Csr &A, Sell &S, int slot, cudaStream_t st)
 {
     S.n = A.n;
     S.nslices = (int)ceil_div(A.n, 32);
@@ -339,11 +368,14 @@ int csr_to_sell(const Csr &A, Sell &S, cudaStream_t st)
     HM_CUDA(cudaMemsetAsync(S.sptr + S.nslices, 0, sizeof(long long), st));
     HM_CUDA(cub::DeviceScan::ExclusiveSum(t, tmp, S.sptr, S.sptr,
                                           S.nslices + 1, st));
-    long long len = 0;
-    HM_CUDA(cudaMemcpyAsync(&len, S.sptr + S.nslices, sizeof(long long),
-                            cudaMemcpyDeviceToHost, st));
-    HM_CUDA(cudaStreamSynchronize(st));
     dfree(t);
+    return read_back(slot, S.sptr + S.nslices, 2, st);
+}
+
+int sell_fill(const Csr &A, Sell &S, int slot, cudaStream_t st)
+{
+    long long len = 0;
+    memcpy(&len, pinned_words() + slot, sizeof(len));
     S.len = len;
     S.col = (int *)dalloc(sizeof(int) * (len > 0 ? len : 1));
     S.val = (double *)dalloc(sizeof(double) * (len > 0 ? len : 1));
@@ -354,7 +386,14 @@ int csr_to_sell(const Csr &A, Sell &S, cudaStream_t st)
     return HMFEM_OK;
 }
 
-int sell_fill_lowp(Sell &S, bool f32, bool bf16, cudaStream_t st)
+int csr_to_sell(const Csr &A, Sell &S, cudaStream_t st)
+{
+    HM_CHECK(sell_layout(A, S, PIN_SELL, st));
+    HM_CUDA(cudaStreamSynchronize(st));
+    return sell_fill(A, S, PIN_SELL, st);
+}
+
+int sell_lowp(Sell &S, bool f32, bool bf16, int *bad, cudaStream_t st)
 {
     if (f32 && !S.val32) S.val32 = (float *)dalloc(sizeof(float) * (S.len > 0 ? S.len : 1));
     if (bf16 && !S.val16) S.val16 = (__nv_bfloat16 *)dalloc(2 * (S.len > 0 ? S.len : 1));
@@ -367,21 +406,30 @@ int sell_fill_lowp(Sell &S, bool f32, bool bf16, cudaStream_t st)
     const char *pe = getenv("HMFEM_PACK16");
     if (bf16 && !S.pk && S.len > 0 && !(pe && atoi(pe) == 0)) {
         S.pk = (unsigned *)dalloc(sizeof(unsigned) * S.len);
-        int *bad = (int *)dalloc(sizeof(int));
-        if (!S.pk || !bad) { dfree(S.pk); dfree(bad); S.pk = nullptr; return HMFEM_E_CUDA; }
-        HM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
+        if (!S.pk) return HMFEM_E_CUDA;
         k_pack16<<<nblocks((long)S.nslices * 32, 256), 256, 0, st>>>(
             S.sptr, S.col, S.val16, (long)S.nslices * 32, S.pk, bad);
         HM_LAUNCHED();
-        int hb = 0;
-        HM_CUDA(cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-        HM_CUDA(cudaStreamSynchronize(st));
-        dfree(bad);
-        if (hb) {  // columns too far from their rows: the col + val16 form
-            dfree(S.pk);
-            S.pk = nullptr;
-        }
     }
+    return HMFEM_OK;
+}
+
+void sell_unpack(Sell &S)  // columns too far from their rows: the col + val16 form
+{
+    dfree(S.pk);
+    S.pk = nullptr;
+}
+
+int sell_fill_lowp(Sell &S, bool f32, bool bf16, cudaStream_t st)
+{
+    int *bad = (int *)dalloc(sizeof(int));
+    if (!bad) return HMFEM_E_CUDA;
+    HM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
+    HM_CHECK(sell_lowp(S, f32, bf16, bad, st));
+    HM_CHECK(read_back(PIN_PACK, bad, 1, st));
+    HM_CUDA(cudaStreamSynchronize(st));
+    dfree(bad);
+    if (pinned_words()[PIN_PACK]) sell_unpack(S);
     return HMFEM_OK;
 }
 

@@ -803,12 +803,13 @@ int g7_build(Level &L, int nx, int ny, int nz, bool f32, cudaStream_t st, int *d
     k_g7_extract<<<nb(n), 256, 0, st>>>(nx, ny, nz, L.A.rowptr, L.A.col, L.A.val, g.cf,
                                         g.cf32, dwork);
     HM_LAUNCHED();
-    int bad = 0;
-    HM_CUDA(cudaMemcpyAsync(&bad, dwork, sizeof(int), cudaMemcpyDeviceToHost, st));
-    HM_CUDA(cudaStreamSynchronize(st));
-    if (bad) { g7_free(g); return HMFEM_OK; }
     L.g7 = g;
-    return HMFEM_OK;
+    return read_back(PIN_G7, dwork, 1, st);
+}
+
+void g7_settle(Level &L)
+{
+    if (L.g7.cf && pinned_words()[PIN_G7]) g7_free(L.g7);
 }
 
 int g19_lowp(Grid19 &g, int n, bool f32, bool bf16, cudaStream_t st)
