@@ -14,6 +14,7 @@ namespace hm {
 
 thread_local std::vector<KRec> *t_kprof = nullptr;
 thread_local int t_nopdl = 0;
+thread_local int t_pdl_blocks = 296;
 thread_local int t_klevel = -1;
 
 int g_pdl = [] {
@@ -1155,6 +1156,7 @@ static int cg_sdir(Solver &s, cudaStream_t st)
 
 int cg_init(Solver &s, cudaStream_t st)
 {
+    t_pdl_blocks = pdl_blocks_for(s.lv[0].A.n);
     Level &L0 = s.lv[0];
     const int n = L0.A.n;
     if (s.use_g7(0)) {
@@ -1173,6 +1175,7 @@ int cg_init(Solver &s, cudaStream_t st)
 
 int cg_iteration(Solver &s, cudaStream_t st)
 {
+    t_pdl_blocks = pdl_blocks_for(s.lv[0].A.n);
     t_klevel = -1;
     Level &L0 = s.lv[0];
     const int n = L0.A.n;

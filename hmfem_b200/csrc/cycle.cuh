@@ -42,6 +42,16 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
     } while (0)
 
 extern int g_pdl;  // 0: plain stream order (HMFEM_PDL=0)
+// Only launches of a limited size are scheduled early: a small kernel gains
+// its launch latency, but the blocks of a large one that wait on the SMs take
+// room from the kernel that still runs.  One CG iteration (us) with every
+// launch early / none / up to 296 blocks: 256^3 reduced precision 1304 / 1237
+// / 1228, 256^3 FP64 2375 / 2302 / 2296, 128^3 reduced 297 / 289 / 282, 32^3
+// FP64 67 / 77 / 67.  Where level 0 itself is one pass of short kernels (up to
+// ~180000 rows) the limit lies above it: the coupled run at 210x42x20 takes
+// 199 ms with 296, 191 with 700, and 128^3 15.1 against 14.9 with 700.
+extern thread_local int t_pdl_blocks;
+inline int pdl_blocks_for(long n0) { return n0 <= 180000 ? 704 : 296; }
 // set while capturing into a conditional node's body (plain stream order
 // there: such bodies hold kernel nodes without programmatic edges)
 extern thread_local int t_nopdl;
@@ -76,7 +86,7 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = (g_pdl && !t_nopdl) ? 1 : 0;
+    cfg.numAttrs = (g_pdl && !t_nopdl && grid <= t_pdl_blocks) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // error: cudaGetLastError
     if (t_kprof) {
         cudaEventRecord(rec.e1, st);
