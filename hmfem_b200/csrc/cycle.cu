@@ -333,6 +333,161 @@ k_cheb_step(const long long *__restrict__ sptr, const int *__restrict__ scol,
                                                   dout, r, u, last, PlainLd{});
 }
 
+// ---- the same rows by teams of warps (levels that leave the chip idle) -----
+//
+// A row per thread walks its entries in rounds of dependent loads (entry,
+// gathered value), 5 us for a level of a few thousand rows as for one of a
+// hundred thousand, while most of the chip's warps are missing.  Here a block
+// of W warps takes one 32-row slice: the warps load the slice's entries and
+// gather side by side, W x 8 of a row in flight, and leave the factors in
+// shared memory (FP64: the rounded products); warp 0 then adds each row up in
+// stored order, so the bits are those of the row-per-thread kernels.
+// Measured, one CG iteration (us): 87x61x75 FP64 178 -> 172 (25916 rows),
+// 128^3 reduced 282 -> 275 (17408), 210x42x20 reduced 103 -> 99 (11550), 256^3
+// reduced 1228 -> 1214 (17248).
+template <class T, int W> struct TeamMem {
+    T a[8 * W][32];
+    T x[sizeof(T) == 4 ? 8 * W : 1][32];
+};
+
+// t -/+ the row sum; valid in warp 0.  Every thread of the block calls it.
+template <class T, class M, bool SUB, int W>
+__device__ __forceinline__ T team_row(T t, TeamMem<T, W> &S, const int *__restrict__ scol,
+                                      const M *__restrict__ sval, long long base, int wd, int row,
+                                      const T *__restrict__ x)
+{
+    using A = Ar<T>;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int k0 = 0; k0 < wd; k0 += 8 * W) {
+        T a[8], xv[8];
+        int c[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int k = k0 + w + W * q;
+            const long long o = base + 32LL * k + lane;
+            if constexpr (std::is_same<M, Pk16>::value) {
+                const unsigned e = k < wd ? __ldg(&sval[o].w) : 0u;
+                a[q] = (T)__uint_as_float(e << 16);
+                c[q] = row + ((int)e >> 16);
+            } else {
+                a[q] = k < wd ? (T)ld(sval, o) : (T)0;
+                c[q] = k < wd ? scol[o] : 0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) xv[q] = k0 + w + W * q < wd ? x[c[q]] : (T)0;
+        if (k0 > 0) __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            if constexpr (sizeof(T) == 4) {
+                S.a[w + W * q][lane] = a[q];
+                S.x[w + W * q][lane] = xv[q];
+            } else {
+                S.a[w + W * q][lane] = A::mul(a[q], xv[q]);
+            }
+        }
+        __syncthreads();
+        if (w == 0) {
+            const int m = min(8 * W, wd - k0);
+#pragma unroll 8
+            for (int k = 0; k < m; k++) {
+                if constexpr (sizeof(T) == 4)
+                    t = SUB ? nmul_add(t, S.a[k][lane], S.x[k][lane])
+                            : pmul_add(t, S.a[k][lane], S.x[k][lane]);
+                else
+                    t = SUB ? A::sub(t, S.a[k][lane]) : A::add(t, S.a[k][lane]);
+            }
+        }
+    }
+    return t;
+}
+
+// WHAT: 0-2 the Chebyshev steps of k_cheb_step's MODE, 3 k_cheb0, 4 k_pre
+template <class T, class M, int W, int WHAT>
+__global__ void __launch_bounds__(32 * W)
+k_team(const long long *__restrict__ sptr, const int *__restrict__ scol,
+       const M *__restrict__ sval, int n, const T *__restrict__ f, const T *__restrict__ dinv,
+       T c1, T c2, const T *__restrict__ x, T *__restrict__ out, T *__restrict__ rv,
+       T *__restrict__ u, const int *__restrict__ prow, int last, const Ctl *ctl)
+{
+    using A = Ar<T>;
+    __shared__ TeamMem<T, W> S;
+    PDL_ENTRY();
+    const bool over = finished(ctl);  // (looked at once the first loads are on their way)
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nsl = (n + 31) >> 5;
+    for (int q = blockIdx.x; q < nsl; q += gridDim.x) {
+        const long long base = sptr[q];
+        const int wd = (int)((sptr[q + 1] - base) >> 5);
+        const int i = 32 * q + lane;
+        const bool own = w == 0 && i < n;
+        // the row's own values, while the entries are on their way
+        T fi = (T)0, di = (T)0, xi = (T)0, ri = (T)0, ui = (T)0;
+        int pc = 0;
+        if (own) {
+            if (WHAT == 0 || WHAT >= 3) fi = f[i];
+            if (WHAT <= 3) di = dinv[i];
+            if (WHAT <= 2) xi = x[i];
+            if (WHAT == 1 || WHAT == 2) { ri = rv[i]; ui = u[i]; }
+            if (WHAT == 4) pc = prow[i + 1] - prow[i];
+        }
+        if (over) return;
+        const T t = team_row<T, M, (WHAT >= 3), W>(WHAT >= 3 ? fi : (T)0, S, scol, sval, base, wd, i,
+                                                   x);
+        if (own) {
+            if (WHAT <= 2) {
+                const T rn = WHAT == 0 ? mul_sub(di, fi, di, t) : nmul_add(ri, di, t);
+                const T dn = mul_add(c1, xi, c2, rn);
+                u[i] = WHAT == 0 ? A::add(xi, dn)
+                     : WHAT == 1 ? A::add(A::add(ui, xi), dn) : A::add(ui, dn);
+                if (!last) {
+                    rv[i] = rn;
+                    out[i] = dn;
+                }
+            } else if (WHAT == 3) {
+                rv[i] = A::mul(di, t);
+                out[i] = A::mul(A::mul(c1, t), di);
+            } else {
+                out[i] = pc == 1 ? t : A::div(t, (T)pc);
+            }
+        }
+        __syncthreads();  // S is free for the next slice
+    }
+}
+
+// Warps per slice for a level of n rows: up to 16 warps per SM (18944 rows by
+// four, 37888 by two).  With up to 48 a level of 62720 rows came out slower
+// (160x96x64: 192 -> 211 us an iteration), eight per slice no faster than four.
+static int team_warps(int n)
+{
+    const long sl = (n + 31) / 32;
+    return sl * 4 <= 148L * 16 ? 4 : sl * 2 <= 148L * 16 ? 2 : 1;
+}
+
+// one of k_team's kernels where teams pay (false: the caller launches the
+// row-per-thread one)
+template <class T, class M, int WHAT>
+static bool launch_team(cudaStream_t st, const Sell &S, const M *vals, int n, const T *f,
+                        const T *dinv, T c1, T c2, const T *x, T *out, T *rv, T *u,
+                        const int *prow, int last, const Ctl *ctl)
+{
+    const int w = team_warps(n), nsl = (n + 31) / 32;
+    // HMFEM_TEAM=0: a row per thread on every level (a check of the teams)
+    const char *on = getenv("HMFEM_TEAM");
+    if (w == 1 || (on && atoi(on) == 0)) return false;
+    auto go = [&](auto kern) {
+        // (many small blocks, but a short kernel: scheduled early)
+        const int limit = t_pdl_blocks;
+        t_pdl_blocks = nsl;
+        launch_pdl(kern, nsl, 32 * w, st, S.sptr, S.col, vals, n, f, dinv, c1, c2, x, out, rv, u,
+                   prow, last, ctl);
+        t_pdl_blocks = limit;
+    };
+    if (w == 4) go(k_team<T, M, 4, WHAT>);
+    else go(k_team<T, M, 2, WHAT>);
+    return true;
+}
+
 // ---- multicolour Gauss-Seidel (coarse levels) ---------------------------
 
 // Forward sweep from zero, first colour: u_i = f_i / a_ii on colour 0,
@@ -971,14 +1126,27 @@ static int cycle_t(Solver &s, int l, cudaStream_t st, bool dot, bool seeded)
             using M = typename std::remove_const<
                 typename std::remove_pointer<decltype(vals)>::type>::type;
             for (int k = 1; k < K; k++) {
+                const T *din = dbuf[(k - 1) & 1];
+                T *dout = dbuf[k & 1];
+                const T c1 = (T)cc.c1[k], c2 = (T)cc.c2[k];
+                const int lst = k == K - 1;
+                if (k == 1 ? launch_team<T, M, 0>(st, L.S, vals, n, f, dv, c1, c2, din, dout, rs, ua,
+                                                  nullptr, lst, ctl)
+                           : launch_team<T, M, 2>(st, L.S, vals, n, f, dv, c1, c2, din, dout, rs, ua,
+                                                  nullptr, lst, ctl)) {
+                    HM_COUNT();
+                    continue;
+                }
                 auto kern = k == 1 ? k_cheb_step<T, M, 0> : k_cheb_step<T, M, 2>;
                 launch_pdl(kern, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, dv,
                            (T)cc.c1[k], (T)cc.c2[k], dbuf[(k - 1) & 1], dbuf[k & 1], rs, ua,
                            (int)(k == K - 1), ctl);
                 HM_COUNT();
             }
-            launch_pdl(k_pre<T, M>, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, ua,
-                       L.P.rowptr, rs, ctl);
+            if (!launch_team<T, M, 4>(st, L.S, vals, n, f, (const T *)nullptr, (T)0, (T)0, ua, rs,
+                                      (T *)nullptr, (T *)nullptr, L.P.rowptr, 0, ctl))
+                launch_pdl(k_pre<T, M>, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, ua,
+                           L.P.rowptr, rs, ctl);
             HM_COUNT();
         });
     } else if (g7) {
@@ -1036,10 +1204,23 @@ static int cycle_t(Solver &s, int l, cudaStream_t st, bool dot, bool seeded)
         with_vals<T>(s, L.S, l, [&](auto vals) {
             using M = typename std::remove_const<
                 typename std::remove_pointer<decltype(vals)>::type>::type;
-            launch_pdl(k_cheb0<T, M>, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, dv,
-                       (T)cc.ith, ua, rs, dbuf[0], ctl);
+            if (!launch_team<T, M, 3>(st, L.S, vals, n, f, dv, (T)cc.ith, (T)0, ua, dbuf[0], rs,
+                                      (T *)nullptr, nullptr, 0, ctl))
+                launch_pdl(k_cheb0<T, M>, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, dv,
+                           (T)cc.ith, ua, rs, dbuf[0], ctl);
             HM_COUNT();
             for (int k = 1; k < K; k++) {
+                const T *din = dbuf[(k - 1) & 1];
+                T *dout = dbuf[k & 1];
+                const T c1 = (T)cc.c1[k], c2 = (T)cc.c2[k];
+                const int lst = k == K - 1;
+                if (k == 1 ? launch_team<T, M, 1>(st, L.S, vals, n, f, dv, c1, c2, din, dout, rs, ua,
+                                                  nullptr, lst, ctl)
+                           : launch_team<T, M, 2>(st, L.S, vals, n, f, dv, c1, c2, din, dout, rs, ua,
+                                                  nullptr, lst, ctl)) {
+                    HM_COUNT();
+                    continue;
+                }
                 auto kern = k == 1 ? k_cheb_step<T, M, 1> : k_cheb_step<T, M, 2>;
                 launch_pdl(kern, nb(n), 256, st, L.S.sptr, L.S.col, vals, n, f, dv,
                            (T)cc.c1[k], (T)cc.c2[k], dbuf[(k - 1) & 1], dbuf[k & 1], rs, ua,

@@ -21,6 +21,34 @@ template <> struct Ar<float> {
     static __device__ __forceinline__ float div(float a, float b) { return a / b; }
 };
 
+// The products and sums of the level kernels with the contraction spelled
+// out, so that FP32 rounds as there whatever the code around it: x y - z w
+// and x y + z w take the first product exactly, t - x y the only one.
+template <class T> __device__ __forceinline__ T mul_sub(T x, T y, T z, T w)
+{
+    using A = Ar<T>;
+    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, -__fmul_rn(z, w));
+    else return A::sub(A::mul(x, y), A::mul(z, w));
+}
+template <class T> __device__ __forceinline__ T mul_add(T x, T y, T z, T w)
+{
+    using A = Ar<T>;
+    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, __fmul_rn(z, w));
+    else return A::add(A::mul(x, y), A::mul(z, w));
+}
+template <class T> __device__ __forceinline__ T nmul_add(T t, T x, T y)
+{
+    using A = Ar<T>;
+    if constexpr (sizeof(T) == 4) return __fmaf_rn(-x, y, t);
+    else return A::sub(t, A::mul(x, y));
+}
+template <class T> __device__ __forceinline__ T pmul_add(T t, T x, T y)
+{
+    using A = Ar<T>;
+    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, t);
+    else return A::add(t, A::mul(x, y));
+}
+
 __device__ __forceinline__ double ld(const double *p, long long i) { return p[i]; }
 __device__ __forceinline__ float ld(const float *p, long long i) { return __ldg(p + i); }
 __device__ __forceinline__ float ld(const __nv_bfloat16 *p, long long i) { return __bfloat162float(p[i]); }

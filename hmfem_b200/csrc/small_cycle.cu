@@ -83,34 +83,6 @@ struct ScArgs {
 // through the finer level's P (u).
 enum ScMask { SC_A, SC_R, SC_P, SC_MASKS };
 
-// The products and sums of the level kernels with the contraction spelled
-// out, so that FP32 rounds as there whatever the code around it: x y - z w
-// and x y + z w take the first product exactly, t - x y the only one.
-template <class T> __device__ __forceinline__ T mul_sub(T x, T y, T z, T w)
-{
-    using A = Ar<T>;
-    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, -__fmul_rn(z, w));
-    else return A::sub(A::mul(x, y), A::mul(z, w));
-}
-template <class T> __device__ __forceinline__ T mul_add(T x, T y, T z, T w)
-{
-    using A = Ar<T>;
-    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, __fmul_rn(z, w));
-    else return A::add(A::mul(x, y), A::mul(z, w));
-}
-template <class T> __device__ __forceinline__ T nmul_add(T t, T x, T y)
-{
-    using A = Ar<T>;
-    if constexpr (sizeof(T) == 4) return __fmaf_rn(-x, y, t);
-    else return A::sub(t, A::mul(x, y));
-}
-template <class T> __device__ __forceinline__ T pmul_add(T t, T x, T y)
-{
-    using A = Ar<T>;
-    if constexpr (sizeof(T) == 4) return __fmaf_rn(x, y, t);
-    else return A::add(t, A::mul(x, y));
-}
-
 // t -/+ sum of a row's entries in stored order; o: the row's first entry, 32
 // apart; eight (FP64: four) at a time so that the gathers overlap
 template <class T, class M, bool SUB, class X>

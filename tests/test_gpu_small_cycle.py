@@ -18,8 +18,9 @@ FORMS = {"fp64": dict(), "fp32": dict(precision=1), "bf16": dict(precision=1, bf
          "schur": dict(precision=1, bf16_from=1, schur0=1)}
 
 
-def _run(p, monkeypatch, on, **opt):
+def _run(p, monkeypatch, on, team="1", **opt):
     monkeypatch.setenv("HMFEM_SMALL_CYCLE", on)
+    monkeypatch.setenv("HMFEM_TEAM", team)
     s = gpu.Solver(tol=1e-9, **opt)
     s.assemble(p)
     s.setup()
@@ -55,3 +56,16 @@ def test_degrees_and_level_ranges(degree, cheb_from, direct, monkeypatch):
         b = _run(p, monkeypatch, "0", **opt, **prec)
         assert a[3] and not b[3]
         assert a[2] == b[2] and np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("shape", [(17, 9, 7), (48, 48, 48), (91, 61, 63), (120, 96, 80)])
+def test_teams_give_the_row_kernels_bits(shape, form, monkeypatch):
+    """Warps sharing a slice's loads (levels of up to ~38000 rows) against a
+    row per thread, with the one-launch form off so that every level has its
+    kernels."""
+    p = make_problem(*shape, log10k=(-14.0, 1.0, 2.0), seed=shape[1])
+    a = _run(p, monkeypatch, "0", team="1", **FORMS[form])
+    b = _run(p, monkeypatch, "0", team="0", **FORMS[form])
+    assert a[2] == b[2]
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
