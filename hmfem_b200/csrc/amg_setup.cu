@@ -726,20 +726,27 @@ int ensure_p(Level &L, cudaStream_t st)
     return HMFEM_OK;
 }
 
-// Per host thread: the stream that forms level 1's split while level 0's
+// Per host thread: the stream of the setup's side work -- level 1's split, formed while level 0's
 // Galerkin product runs (the split depends only on the grid's shape).  Its
 // kernels are a latency-bound wavefront of small launches, so the stream
 // has the highest priority: their blocks are scheduled between the
 // bandwidth-bound blocks of the main stream instead of after them.
-static cudaStream_t side_stream()
+cudaStream_t side_stream()
 {
-    static thread_local cudaStream_t t_side = nullptr;
-    if (!t_side) {
+    struct Side {
+        cudaStream_t st = nullptr;
+        ~Side()
+        {
+            if (st) cudaStreamDestroy(st);  // with its thread
+        }
+    };
+    static thread_local Side side;
+    if (!side.st) {
         int least = 0, greatest = 0;
         cudaDeviceGetStreamPriorityRange(&least, &greatest);
-        cudaStreamCreateWithPriority(&t_side, cudaStreamNonBlocking, greatest);
+        cudaStreamCreateWithPriority(&side.st, cudaStreamNonBlocking, greatest);
     }
-    return t_side;
+    return side.st;
 }
 
 int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *dwork,

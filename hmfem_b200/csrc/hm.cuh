@@ -195,6 +195,7 @@ int launch_spmv(const Sell &S, const double *x, double *y, cudaStream_t st);
 // (rap_stencil.cu), bit-identical to the generic kernels.
 int amg_coarsen(Level &L, Level &C, cudaStream_t st, int *err_dev,
                 const int *grid3 = nullptr, bool schur = false);
+cudaStream_t side_stream();  // amg_setup.cu
 // the rest of the hierarchy below level l >= 1 of at most 512 rows, in one
 // launch (amg_tail.cu): appends the levels to lv, *levels of them (0: the
 // general path has to go on)

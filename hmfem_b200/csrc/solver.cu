@@ -169,7 +169,7 @@ static int gj_launches(int n, double *a, double *b, int *err, cudaStream_t st)
     return HMFEM_OK;
 }
 
-int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st)
+int dense_factor(const Csr &A, double *Lf, double *tmp, int *err, cudaStream_t st)
 {
     const int n = A.n;
     if (n <= 0) return HMFEM_OK;
@@ -177,8 +177,6 @@ int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st)
         set_last_error("dense coarse solve: level too large", __FILE__, __LINE__);
         return HMFEM_E_ARG;
     }
-    double *tmp = (double *)dalloc(sizeof(double) * (size_t)n * n);
-    if (!tmp) return HMFEM_E_CUDA;
     const int launches = (int)ceil_div(n, kGjBlock);
     // after the last launch the inverse must land in Lf: start in the other buffer
     double *a = (launches & 1) ? tmp : Lf, *b = (launches & 1) ? Lf : tmp;
@@ -188,9 +186,27 @@ int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st)
     else if (n <= 256) HM_CHECK(gj_launches<8>(n, a, b, err, st));
     else if (n <= 384) HM_CHECK(gj_launches<12>(n, a, b, err, st));
     else HM_CHECK(gj_launches<16>(n, a, b, err, st));
-    dfree(tmp);  // to the solver's cache, whose blocks are reused on its stream only
     return HMFEM_OK;
 }
+
+// The coarse inverse runs on the side stream as soon as its level exists,
+// beside the launch that makes the levels below and the solve-phase forms:
+// both are serial chains that leave the chip idle (0.25 ms each).
+struct DenseJob {
+    int level = -1;
+    double *tmp = nullptr;
+    cudaEvent_t done = nullptr;
+    ~DenseJob()
+    {
+        if (done) {
+            cudaEventSynchronize(done);  // (already waited for unless setup failed)
+            cudaEventDestroy(done);
+        }
+        dfree(tmp);
+    }
+};
+
+static int dense_start(Solver &s, DenseJob &job, int l);
 
 // constant values of the boundary faces (n = 0: given by the caller)
 struct FaceFill {
@@ -454,6 +470,29 @@ int level_forms(Solver &s, int k0, int k1, int dense, cudaStream_t st)
     return HMFEM_OK;
 }
 
+static int dense_start(Solver &s, DenseJob &job, int l)
+{
+    const Level &L = s.lv[l];
+    const long n = L.A.n;
+    if (job.level >= 0 || n > s.opt.coarse_direct || n > kDenseMax) return HMFEM_OK;
+    HM_ALLOC(s.dense_L, double, n * n);
+    HM_ALLOC(job.tmp, double, n * n);
+    int *err = s.dwork + 10;
+    HM_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s.st));
+    cudaEvent_t ready;
+    HM_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    HM_CUDA(cudaEventRecord(ready, s.st));
+    cudaStream_t side = side_stream();
+    HM_CUDA(cudaStreamWaitEvent(side, ready, 0));
+    cudaEventDestroy(ready);
+    const int rc = dense_factor(L.A, s.dense_L, job.tmp, err, side);
+    HM_CUDA(cudaEventCreateWithFlags(&job.done, cudaEventDisableTiming));
+    HM_CUDA(cudaEventRecord(job.done, side));
+    HM_CHECK(rc);
+    job.level = l;
+    return HMFEM_OK;
+}
+
 int setup(Solver &s)
 {
     if (s.lv.empty() || !s.lv[0].A.col) {
@@ -473,6 +512,7 @@ int setup(Solver &s)
     HM_PHASE("setup: free", st);
     s.lv.reserve(s.opt.max_levels + 1);
     // level loop (amg.h:1186-1213)
+    DenseJob dense_job;
     int l = 0;
     long gcnt = s.lv[0].A.n;
     double rel = 0.0;
@@ -492,12 +532,15 @@ int setup(Solver &s)
             HM_ALLOC(L.dinv32, float, L.A.n);
             HM_CHECK(launch_diag_inv(L.A, L.dinv, L.dinv32, st, l == 0 ? s.dwork + 8 : nullptr));
         }
+        // (the first level small enough is the one solved by its inverse)
+        HM_CHECK(dense_start(s, dense_job, l));
         if (!(l < s.opt.max_levels - 1 && gcnt > s.opt.min_coarse && rel < 1.0)) break;
         if (tail_applies(L, l) && !L.tail_matrix) {
             int made = 0;
             HM_CHECK(amg_tail(s.lv, l, s.opt.max_levels, s.opt.min_coarse, s.tail, st, &made));
             HM_PHASE("  small levels", st);
             if (made > 0) {
+                for (int k = 1; k <= made; k++) HM_CHECK(dense_start(s, dense_job, l + k));
                 l += made;
                 gcnt = s.lv[l].A.n;
                 rel = (double)gcnt / (double)s.lv[l - 1].A.n;
@@ -539,19 +582,11 @@ int setup(Solver &s)
         else
             g19_free(s.lv[1].g19);
     }
-    // dense coarse solve on the first level small enough
     s.direct_level = -1;
-    int dense = -1;
-    if (s.opt.coarse_direct > 0) {
-        for (int k = 0; k < s.nlevels && dense < 0; k++)
-            if (s.lv[k].A.n <= s.opt.coarse_direct && s.lv[k].A.n <= kDenseMax) dense = k;
-        if (dense >= 0) {
-            const long n = s.lv[dense].A.n;
-            HM_ALLOC(s.dense_L, double, n * n);
-            HM_CUDA(cudaMemsetAsync(s.dwork, 0, sizeof(int), st));
-            HM_CHECK(dense_factor(s.lv[dense].A, s.dense_L, s.dwork, st));
-            HM_CHECK(read_back(PIN_DENSE, s.dwork, 1, st));
-        }
+    const int dense = dense_job.level;
+    if (dense >= 0) {
+        HM_CUDA(cudaStreamWaitEvent(st, dense_job.done, 0));
+        HM_CHECK(read_back(PIN_DENSE, s.dwork + 10, 1, st));
     }
     // solve-phase formats and vectors of the levels the cycle visits (those
     // below the coarse solve get theirs when something asks for them)

@@ -124,7 +124,7 @@ int cg_precondition(Solver &s, cudaStream_t st);
 int cg_final_residual(Solver &s, cudaStream_t st);
 int launch_smoother_diag(const Csr &A, int kind, double *dsm, float *dsm32,
                          cudaStream_t st);
-int dense_factor(const Csr &A, double *Lf, int *err, cudaStream_t st);
+int dense_factor(const Csr &A, double *Lf, double *tmp, int *err, cudaStream_t st);
 int time_kernel(Solver &s, int which, int l, int reps, float *ms, double *bytes);
 int small_cycle_build(Solver &s, cudaStream_t st);
 int small_cycle(Solver &s, const double *c1, const double *c2, double ith, const Ctl *ctl,
