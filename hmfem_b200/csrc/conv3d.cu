@@ -761,9 +761,11 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
 // taps in its columns: with 16 -> 16 channels 48 x 144 useful entries of
 // 128 x 144 for 16 cells, against 16 x 16 of 128 x 16 for one tap per MMA
 // (one tap per CTA, both operands transposed through registers).  Measured
-// against that form: 16 -> 16 at 128^3 2707 -> 113 us, 48 -> 16 3814 -> 250,
-// 96 -> 32 at 64^3 1335 -> 104, 64 -> 64 at 32^3 125 -> 32.  What bounds it
-// now are the group copies (16 -> 16: 12 groups for each 128 x 144 MMA).
+// against that form: 16 -> 16 at 128^3 2707 -> 110 us, 48 -> 16 3814 -> 204,
+// 96 -> 32 at 64^3 1335 -> 80, 64 -> 64 at 32^3 125 -> 26.  Bound by the
+// operands' shared-memory reads (16 -> 16) or the copies (96 -> 32): a copy
+// brings all slabs of one shift (one per group took 104 us at 96 -> 32), and
+// bulk copies by row with zeros stored around them were slower (162).
 //
 // A step is 32 x BY cells of one z plane.  A group is one slab (8 channels)
 // of a step, BY rows of 32 cells, 16 bytes a cell: an MN-major operand
@@ -784,6 +786,7 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
 struct WgPlan {
     int flip;              // 0: M = x, N = dy; 1: M = dy, N = x
     int ms, gm, gmax;      // M side: slabs, groups (3 ms), groups per stage
+    int mb;                // groups per copy: divides ms and 16
     int mblk, parts;       // M blocks; parts = mblk x (N slabs / NS)
     int cin, cout;
     int nxc, nyb, zl, nzc; // 32-cell columns, BY-row blocks, z planes per item, items along z
@@ -799,7 +802,7 @@ struct WgCfg {
     static constexpr int COLS = 72 * NS;       // columns of D: 3 planes x GN x 8
     static constexpr int TCOLS = COLS <= 256 ? 256 : 512;
     static constexpr int RM = BY == 4 ? 3 : 4;
-    static constexpr int RN = BY == 4 ? 6 : NS == 4 ? 8 : 7;
+    static constexpr int RN = BY == 4 ? 10 : NS == 4 ? 8 : 7;
     static constexpr int kBytes(int gmax) { return (RM * gmax + RN * GN) * SP + 256; }
 };
 
@@ -843,10 +846,10 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
     if (warp == 4) {
         Ring rm{0, 0u}, rn{0, 0u};
         long mseq = 0, nseq = 0;
-        // this lane's group: of the M side (x shift, slab), of an N plane
-        // (y shift, slab)
-        const int gi = (g0 + lane) / p.ms, gs = (g0 + lane) % p.ms;
-        const int nj = lane / NS, nslab = s0 + lane % NS;
+        // a lane's copy: mb groups (slabs of one x shift) of the M side, the NS
+        // slabs of one y shift of an N plane
+        const int gl = lane * p.mb;
+        const int gi = (g0 + gl) / p.ms, gs = (g0 + gl) % p.ms;
         bool ok = true;
         for (long it = idx; it < items && ok; it += p.per) {
             const int xc = (int)(it % p.nxc), yb = (int)((it / p.nxc) % p.nyb),
@@ -860,9 +863,9 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
                 }
                 if (lane == 0) mbar_expect_tx_only(&full_n[rn.i], GN * SP);
                 __syncwarp();
-                if (lane < GN)
-                    tma_load_4d(smem_u32(nring + (rn.i * GN + lane) * SP), &tm_n, 256 * xc,
-                                BY * yb + nj - 1, z, nslab, &full_n[rn.i]);
+                if (lane < 3)
+                    tma_load_4d(smem_u32(nring + (rn.i * GN + lane * NS) * SP), &tm_n, 256 * xc,
+                                BY * yb + lane - 1, z, s0, &full_n[rn.i]);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full_n[rn.i]);
                 rn.next(RN);
@@ -875,8 +878,8 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
                 }
                 if (lane == 0) mbar_expect_tx_only(&full_m[rm.i], (uint32_t)(gmc * SP));
                 __syncwarp();
-                if (lane < gmc)
-                    tma_load_4d(smem_u32(mring + rm.i * mstage + lane * SP), &tm_m,
+                if (gl < gmc)
+                    tma_load_4d(smem_u32(mring + rm.i * mstage + gl * SP), &tm_m,
                                 256 * xc + 8 * (gi - 1), BY * yb, z - 1, gs, &full_m[rm.i]);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full_m[rm.i]);
@@ -1228,6 +1231,7 @@ int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, i
     p.ms = cm / 8;
     p.gm = 3 * p.ms;
     p.gmax = p.gm < 16 ? p.gm : 16;
+    p.mb = p.ms % 8 == 0 ? 8 : p.ms % 4 == 0 ? 4 : 2;
     p.mblk = (p.gm + 15) / 16;
     p.parts = p.mblk * (cn / 8 / NS);
     p.nxc = (nx + 31) / 32;
@@ -1262,7 +1266,7 @@ int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, i
                                     (cuuint64_t)ch[i] / 8};
         const cuuint64_t strides[3] = {(cuuint64_t)nx * 16, (cuuint64_t)nx * ny * 16,
                                        (cuuint64_t)nx * ny * nz * 16};
-        const cuuint32_t box[4] = {256, (cuuint32_t)BY, 1, 1};
+        const cuuint32_t box[4] = {256, (cuuint32_t)BY, 1, (cuuint32_t)(i == 0 ? p.mb : NS)};
         const int rc = encode_bf16_map(&tm[i], base[i], 4, dims, strides, box);
         if (rc != HMFEM_OK) return rc;
     }
