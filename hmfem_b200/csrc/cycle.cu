@@ -850,7 +850,13 @@ __global__ void __launch_bounds__(256)
 k_sdir(int n, double *__restrict__ s, const T *__restrict__ z, Ctl *ctl)
 {
     PDL_ENTRY();
-    if (finished(ctl)) return;
+    // the iteration's last kernel tells the host how far the solve is
+    const bool tell = blockIdx.x == 0 && threadIdx.x == 0 && ctl->host;
+    if (finished(ctl)) {
+        if (tell) *ctl->host = -1;
+        return;
+    }
+    if (tell) *ctl->host = ctl->iters;
     const double be = ctl->beta;
     // two cells per thread, 16-byte accesses to s (same operations per cell)
     using Z2 = typename std::conditional<std::is_same<T, double>::value, double2, float2>::type;

@@ -126,6 +126,9 @@ struct Ctl {
     double rr, bb, trr, tol2, rz_old;
     int done, check, iters, status, max_iter, stop_rule, nrep, pad;
     unsigned tickets[16];
+    // pinned word of the host that solves: the iterations done, -1 once the
+    // solve is over (null: nobody looks)
+    volatile int *host;
 };
 
 // reduction slots (tickets[] index + partial buffer row)
@@ -271,7 +274,7 @@ void set_alloc_context(cudaStream_t st, AllocCache *c);
 void get_alloc_context(cudaStream_t *st, AllocCache **c);
 AllocCache *alloc_cache_new();
 // kPinExtra pinned bytes of the cache's owner (null when there are none)
-constexpr size_t kPinExtra = 4096;
+constexpr size_t kPinExtra = 64;
 void *pinned_extra(AllocCache *c);
 void alloc_cache_release(AllocCache *c);
 

@@ -66,7 +66,7 @@ struct Solver {
     bool zdots_done = false;
     Ctl *ctl = nullptr;
     Ctl ctl_init{};  // host copy of the control block a solve starts from
-    Ctl *ctl_host = nullptr;  // pinned, 2 slots
+    volatile int *progress = nullptr;  // pinned: Ctl::host of a solve
     double *part = nullptr;
     int *dwork = nullptr;
     SmallCycle small;
