@@ -221,6 +221,7 @@ struct ConvPlan {
 
 constexpr int kConvThreads = 192;  // warps 0-3 epilogue, 4 TMA producer, 5 MMA
 constexpr int kEpilogue = 128;
+constexpr int kMaxSmem = 227 * 1024;  // dynamic shared memory a block may have
 constexpr unsigned kWResMax = 64 * 1024;  // resident weights (all chunks) up to this size
 constexpr unsigned kBarBytes = 128;       // mbarriers (ns, nb <= 4), TMEM slot, abort flag
 constexpr int kMaxPlaneX = 1024;          // widest grid a plane-mode tile spans
@@ -1199,7 +1200,8 @@ int launch_fwd(const void *in, const void *w, const float *bias, void *out, int 
         const int rc = encode_bf16_map(&tm_w, w, 3, dims, strides, box);
         if (rc != HMFEM_OK) return rc;
     }
-    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem_bytes));
+    // (the attribute is the process's: the same value from every thread)
+    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     const long tiles = (long)p.ntx * p.nty * p.ntz;
     const int grid = (int)(tiles < nsm ? tiles : nsm);
     k<<<grid, kConvThreads, p.smem_bytes, st>>>((const __nv_bfloat16 *)in, tm_w, bias,
@@ -1274,7 +1276,7 @@ int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, i
     // the A operand's 16 groups from the last M stage stay inside the buffer
     static_assert(16 * C::SP <= C::RN * C::GN * C::SP, "operand overrun");
     auto k = k_wgrad<NS, BY>;
-    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     k<<<(unsigned)(per * p.parts), kConvThreads, bytes, st>>>(tm[0], tm[1], dw, nz, p, err);
     HM_LAUNCHED();
     return HMFEM_OK;

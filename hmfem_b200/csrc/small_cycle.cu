@@ -383,9 +383,10 @@ template <class T, class M>
 cudaError_t sc_launch(const ScArgs &a, int ctas, size_t smem, bool pdl, cudaStream_t st,
                       int *active)
 {
-    cudaError_t e = cudaFuncSetAttribute(k_small_cycle<T, M>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && ctas > 8)
+    // (the attributes are the process's: the same values from every thread)
+    cudaError_t e = cudaFuncSetAttribute(
+        k_small_cycle<T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScSmem);
+    if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_small_cycle<T, M>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;

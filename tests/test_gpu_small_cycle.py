@@ -69,3 +69,21 @@ def test_teams_give_the_row_kernels_bits(shape, form, monkeypatch):
     b = _run(p, monkeypatch, "0", team="0", **FORMS[form])
     assert a[2] == b[2]
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+def test_threads_with_different_grids():
+    """Solvers whose cluster launches take different amounts of shared
+    memory, captured and launched from eight threads at once."""
+    from hmfem_b200 import batch
+
+    shapes = [(14, 12, 10), (24, 20, 16), (33, 31, 17), (40, 36, 30)]
+    probs = [make_problem(*shapes[i % 4], log10k=(-14.0, 1.0, 2.0), seed=i) for i in range(64)]
+    out = batch.solve_batch(probs, precision=1, tol=1e-9, workers=8)
+    for i in (0, 1, 2, 3):
+        s = gpu.Solver(precision=1, tol=1e-9)
+        s.assemble(probs[i])
+        s.setup()
+        x, st = s.solve()
+        s.close()
+        assert st["iterations"] == out[i][1]["iterations"]
+        assert np.array_equal(x, out[i][0])
