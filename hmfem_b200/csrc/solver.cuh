@@ -40,6 +40,7 @@ struct Solver {
 
     // grid problem (hmfem_assemble)
     bool have_grid = false;
+    int sdim[3] = {0, 0, 0};  // cells per axis of the caller's stencil matrix (0: none)
     int nx = 0, ny = 0, nz = 0;
     double hx = 0, hy = 0, hz = 0, visc = 1;
     int bc[6] = {0, 0, 1, 1, 1, 1};

@@ -653,7 +653,8 @@ k_g19_spmv(G19v<double> g, const double *__restrict__ x, double *__restrict__ y)
 
 // a_cc, a_{c,c+1}, a_{c,c+nx}, a_{c,c+nxy} from the assembled rows (order
 // d,l,c,r,u,t,b over the in-grid neighbours), and a bitwise check of
-// a_{c,c+e} == a_{c+e,c} for the three + directions
+// a_{c,c+e} == a_{c+e,c} for the three + directions.  The rows may be any
+// matrix's (a caller's stencil): an entry is read only where its row holds it
 __global__ void k_g7_extract(int nx, int ny, int nz, const int *__restrict__ rowptr,
                              const int *__restrict__ col, const double *__restrict__ val,
                              double *cf, float *cf32, int *bad)
@@ -667,28 +668,32 @@ __global__ void k_g7_extract(int nx, int ny, int nz, const int *__restrict__ row
         const int pd = o, pl = pd + (j > 0), pc = pl + (i > 0), pr = pc + 1;
         const int pu = pr + (i < nx - 1), pt = pu + (j < ny - 1), pb = pt + (k < nz - 1);
         const int e = pb + (k > 0);
-        bool ok = e == rowptr[s + 1] && col[pc] == (int)s;
+        if (e != rowptr[s + 1]) {  // not this stencil's row: its entries are not read
+            atomicOr(bad, 1);
+            continue;
+        }
+        bool ok = col[pc] == (int)s;
         const double vc = val[pc];
         double vr = 0.0, vu = 0.0, vt = 0.0;
         if (i < nx - 1) {
             vr = val[pr];
             const long q = s + 1;
             const int oq = rowptr[q] + (j > 0);  // its l entry
-            ok = ok && col[pr] == (int)q && col[oq] == (int)s &&
+            ok = ok && col[pr] == (int)q && oq < rowptr[q + 1] && col[oq] == (int)s &&
                  __double_as_longlong(val[oq]) == __double_as_longlong(vr);
         }
         if (j < ny - 1) {
             vu = val[pu];
             const long q = s + nx;
             const int oq = rowptr[q];  // its d entry (first)
-            ok = ok && col[pu] == (int)q && col[oq] == (int)s &&
+            ok = ok && col[pu] == (int)q && oq < rowptr[q + 1] && col[oq] == (int)s &&
                  __double_as_longlong(val[oq]) == __double_as_longlong(vu);
         }
         if (k < nz - 1) {
             vt = val[pt];
             const long q = s + nxy;
             const int oq = rowptr[q + 1] - 1;  // its b entry (last)
-            ok = ok && col[pt] == (int)q && col[oq] == (int)s &&
+            ok = ok && col[pt] == (int)q && oq >= rowptr[q] && col[oq] == (int)s &&
                  __double_as_longlong(val[oq]) == __double_as_longlong(vt);
         }
         const double v4[4] = {vc, vr, vu, vt};
