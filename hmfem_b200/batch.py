@@ -5,15 +5,12 @@ Two drivers:
 * `solve_batch_graph` (the default of the bench): every instance is
   assembled and set up by one of `workers` threads (a solver per instance,
   its own stream and allocation cache), then all instances are solved
-  together by `hmfem_batch_solve`: one CUDA graph holds one CG iteration of
-  every instance -- its V-cycle included -- each on a branch of its own, and
-  is replayed until every instance has converged.  A converged instance's
-  kernels return at once (its own control block): a per-instance
-  convergence mask, each instance stopping at its own tolerance with the
-  result it gives solved alone.
+  together by `hmfem_batch_solve`: each on its own stream, by replaying its
+  own captured CG iteration -- its V-cycle included -- until its own control
+  block says it has converged, so each instance stops at its own tolerance
+  with the result it gives solved alone.
 * `solve_batch`: each worker thread solves whole instances one after
-  another on its own solver (the batch solve of round one, kept for
-  comparison).
+  another on its own solver.
 
 Instances of 24^3..96^3 cells leave most of a B200 idle when run one after
 another (their kernels are small and the setup is launch-bound); the
@@ -112,8 +109,8 @@ def release_pools():
 
 def solve_batch_graph(problems, precision=1, tol=1e-10, workers=8, options=None):
     """Sets every problem up on `workers` threads (each on a solver of the
-    pool kept for these options), then solves them all with one batched
-    graph (hmfem_batch_solve); returns [(x, stats, seconds)] in input order,
+    pool kept for these options), then solves them all side by side, each by
+    its own captured iteration (hmfem_batch_solve); returns [(x, stats, seconds)] in input order,
     seconds = the instance's assembly + setup in its worker + the batched
     solve (which every instance waits for)."""
     opts = dict(precision=precision, tol=tol)

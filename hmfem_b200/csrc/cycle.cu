@@ -13,7 +13,6 @@
 namespace hm {
 
 thread_local std::vector<KRec> *t_kprof = nullptr;
-thread_local int t_nopdl = 0;
 thread_local int t_pdl_blocks = 296;
 thread_local int t_klevel = -1;
 

@@ -80,9 +80,6 @@ extern int g_pdl;  // 0: plain stream order (HMFEM_PDL=0)
 // 199 ms with 296, 191 with 700, and 128^3 15.1 against 14.9 with 700.
 extern thread_local int t_pdl_blocks;
 inline int pdl_blocks_for(long n0) { return n0 <= 180000 ? 704 : 296; }
-// set while capturing into a conditional node's body (plain stream order
-// there: such bodies hold kernel nodes without programmatic edges)
-extern thread_local int t_nopdl;
 
 // Per-launch timing of the solve phase (hmfem_profile_iteration): while
 // t_kprof is set on a host thread, launch_pdl brackets each of its launches
@@ -114,7 +111,7 @@ inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = (g_pdl && !t_nopdl && grid <= t_pdl_blocks) ? 1 : 0;
+    cfg.numAttrs = (g_pdl && grid <= t_pdl_blocks) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // error: cudaGetLastError
     if (t_kprof) {
         cudaEventRecord(rec.e1, st);

@@ -611,7 +611,7 @@ int small_cycle(Solver &s, const double *c1, const double *c2, double ith, const
         using TT = typename std::remove_pointer<decltype(t)>::type;
         using MM = typename std::remove_pointer<decltype(m)>::type;
         rec.fn = (const void *)k_small_cycle<TT, MM>;
-        return sc_launch<TT, MM>(a, S.ctas, S.smem, g_pdl && !t_nopdl, st, nullptr);
+        return sc_launch<TT, MM>(a, S.ctas, S.smem, g_pdl, st, nullptr);
     }));
     if (t_kprof) {
         cudaEventRecord(rec.e1, st);

@@ -787,131 +787,124 @@ static int finish_solve(Solver &s, double *x, int mem, cudaStream_t st, cudaEven
 
 // ---- many solvers solved together -----------------------------------------
 //
-// Every member is set up on its own.  Then ONE CUDA graph solves them all,
-// launched once: for each member a conditional WHILE node whose body is one
-// CG iteration of that member (its V-cycle included) followed by a kernel
-// that keeps the loop going while the member's control block is not done;
-// done is set by the member's own kernels (converged, breakdown, or the
-// iteration cap), so every member iterates exactly as long as it needs and
-// its result is the one a solve on its own gives.  The WHILE nodes are
-// independent, so the members' loops run side by side on the GPU.
+// Every member iterates on its own stream by its own captured iteration, as a
+// solve on its own does, and one host thread keeps all of them supplied: each
+// member's last kernel of an iteration writes its pinned word, and a member
+// whose queue is shorter than check_every gets another launch (6-8 us of host
+// time, so ~20 members can be kept busy at ~150 us per iteration; beyond that
+// the GPU is full anyway).  Bound by the small levels' latency, which the
+// members hide for one another: they run side by side on as many hardware
+// queues as the device has.  One graph with a conditional WHILE node per
+// member was launched once, but its bodies ran mostly one after another and
+// it had to be captured and instantiated anew for every batch.  Grids of 24
+// to 96 cells an edge, the reduced-precision cycle: 4 members 7.9 -> 5.8 ms,
+// 16 members 31.6 -> 23.6, 48 members 65 -> 37.5 (with the largest started
+// first and x copied back while others iterate; 40.2 without).
 
-__global__ void k_while_next(cudaGraphConditionalHandle h, const Ctl *ctl)
+// Sets a member's solve going on its stream.  e0 marks its start.
+static int batch_start(Solver &s, const double *x, int mem, cudaEvent_t *e0)
 {
-    if (threadIdx.x == 0) cudaGraphSetConditional(h, *(volatile const int *)&ctl->done ? 0u : 1u);
+    set_alloc_context(s.st, s.cache);
+    if (!s.setup_done) HM_CHECK(setup(s));
+    const int n = s.lv[0].A.n;
+    if (x) HM_CHECK(upload(s.x, x, n, mem, s.st));
+    else HM_CUDA(cudaMemsetAsync(s.x, 0, sizeof(double) * n, s.st));
+    *s.progress = 0;
+    HM_CHECK(ctl_reset(s, s.st, s.progress));
+    HM_CUDA(cudaEventCreate(e0));
+    HM_CUDA(cudaEventRecord(*e0, s.st));
+    s.ctl_active = true;
+    int rc = cg_init(s, s.st);
+    if (rc == HMFEM_OK && !s.graph) rc = capture_iteration(s);
+    s.ctl_active = false;
+    return rc;
 }
 
 int batch_solve(Solver *const *ss, int m, double *const *x, int mem, hmfem_stats *out)
 {
     if (m <= 0) return HMFEM_OK;
-    cudaStream_t ms;
-    HM_CUDA(cudaStreamCreateWithFlags(&ms, cudaStreamNonBlocking));
-    std::vector<cudaEvent_t> ev(m), ev0(m);
-    int rc = HMFEM_OK;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    std::vector<cudaStream_t> cs(m, nullptr);
-    auto fail = [&](int r) { if (rc == HMFEM_OK) rc = r; };
-    // ---- every member: x, control block, the CG start on its own stream
-    for (int i = 0; i < m && rc == HMFEM_OK; i++) {
+    // the largest first: they iterate longest
+    std::vector<int> order(m);
+    for (int i = 0; i < m; i++) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+        return ss[p]->lv[0].A.n > ss[q]->lv[0].A.n;
+    });
+    struct Member {
+        cudaEvent_t e0 = nullptr;
+        int launched = 0;
+        bool runs = false;
+    };
+    std::vector<Member> mb(m);
+    int rc = HMFEM_OK, ready = 0, left = 0;
+    std::vector<int> status(m, HMFEM_OK);
+    // the final residual, x and the stats of a member that is done, while the
+    // others go on
+    auto finish = [&](int i) {
         Solver &s = *ss[i];
+        mb[i].runs = false;
+        left--;
         set_alloc_context(s.st, s.cache);
-        if (!s.setup_done) { fail(setup(s)); if (rc) break; }
-        const int n = s.lv[0].A.n;
-        if (x && x[i]) { fail(upload(s.x, (const double *)x[i], n, mem, s.st)); }
-        else if (cudaMemsetAsync(s.x, 0, sizeof(double) * n, s.st) != cudaSuccess) fail(HMFEM_E_CUDA);
-        if (rc) break;
-        fail(ctl_reset(s, s.st));
-        if (cudaEventCreate(&ev0[i]) != cudaSuccess) fail(HMFEM_E_CUDA);
-        if (rc) break;
-        cudaEventRecord(ev0[i], s.st);
-        s.ctl_active = true;
-        fail(cg_init(s, s.st));
-        s.ctl_active = false;
-        if (cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess) fail(HMFEM_E_CUDA);
-        if (rc) break;
-        cudaEventRecord(ev[i], s.st);
-        if (cudaStreamWaitEvent(ms, ev[i], 0) != cudaSuccess) fail(HMFEM_E_CUDA);
-    }
-    // ---- one graph: a WHILE node per member
-    std::vector<unsigned long long> body_kernels(m, 0);
-    if (rc == HMFEM_OK && cudaGraphCreate(&graph, 0) != cudaSuccess) fail(HMFEM_E_CUDA);
-    for (int i = 0; i < m && rc == HMFEM_OK; i++) {
-        Solver &s = *ss[i];
-        cudaGraphConditionalHandle h;
-        if (cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault) !=
-            cudaSuccess) {
-            fail(HMFEM_E_CUDA);
-            break;
-        }
-        cudaGraphNodeParams np = {};
-        np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = h;
-        np.conditional.type = cudaGraphCondTypeWhile;
-        np.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, graph, nullptr, 0, &np) != cudaSuccess) {
-            fail(HMFEM_E_CUDA);
-            break;
-        }
-        cudaGraph_t body = np.conditional.phGraph_out[0];
-        if (cudaStreamCreateWithFlags(&cs[i], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaStreamBeginCaptureToGraph(cs[i], body, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-            fail(HMFEM_E_CUDA);
-            break;
-        }
-        const unsigned long long before = t_nlaunch;
-        t_nopdl = 1;
-        s.ctl_active = true;
-        fail(cg_iteration(s, cs[i]));
-        s.ctl_active = false;
-        t_nopdl = 0;
-        k_while_next<<<1, 32, 0, cs[i]>>>(h, s.ctl);
-        HM_COUNT();
-        body_kernels[i] = t_nlaunch - before;
-        g_nlaunch -= body_kernels[i];  // counted per iteration below
-        cudaGraph_t captured = nullptr;
-        if (cudaStreamEndCapture(cs[i], &captured) != cudaSuccess) fail(HMFEM_E_CUDA);
-    }
-    if (rc == HMFEM_OK && cudaGraphInstantiate(&gexec, graph, 0) != cudaSuccess)
-        fail(HMFEM_E_CUDA);
-    // ---- one launch solves every member
-    if (rc == HMFEM_OK) {
-        if (cudaGraphLaunch(gexec, ms) != cudaSuccess) fail(HMFEM_E_CUDA);
-        if (cudaStreamSynchronize(ms) != cudaSuccess) fail(HMFEM_E_CUDA);
-    }
-    // ---- every member: final residual, x, stats
-    int worst = HMFEM_OK;
-    if (rc == HMFEM_OK) {
-        for (int i = 0; i < m; i++) {
+        cudaEvent_t e1;
+        if (cudaEventCreate(&e1) != cudaSuccess) { rc = HMFEM_E_CUDA; return; }
+        status[i] = finish_solve(s, x ? x[i] : nullptr, mem, s.st, mb[i].e0, e1,
+                                 out ? out + i : nullptr);
+        mb[i].e0 = nullptr;
+    };
+    for (unsigned polls = 0; rc == HMFEM_OK && (ready < m || left > 0);) {
+        bool any = false;
+        int done = -1;
+        for (int i = 0; i < m && rc == HMFEM_OK; i++) {
+            if (!mb[i].runs) continue;
             Solver &s = *ss[i];
-            set_alloc_context(s.st, s.cache);
-            cudaEvent_t e1;
-            cudaEventCreate(&e1);
-            // the member's stream after the whole replay
-            cudaEvent_t after;
-            cudaEventCreateWithFlags(&after, cudaEventDisableTiming);
-            cudaEventRecord(after, ms);
-            cudaStreamWaitEvent(s.st, after, 0);
-            cudaEventDestroy(after);
-            const int r = finish_solve(s, x ? x[i] : nullptr, mem, s.st, ev0[i], e1,
-                                       out ? out + i : nullptr);
-            ev0[i] = nullptr;
-            g_nlaunch += (unsigned long long)(s.last.iterations + 1) * body_kernels[i];
-            if (r != HMFEM_OK && worst == HMFEM_OK) worst = r;
+            const int ahead = s.opt.check_every > 0 ? s.opt.check_every : 4;
+            const int at = *s.progress;
+            if (at < 0 || mb[i].launched > s.opt.max_iter + 2 * ahead) {
+                done = i;
+            } else if (mb[i].launched - at < ahead) {
+                if (cudaGraphLaunch(s.gexec, s.st) != cudaSuccess) rc = HMFEM_E_CUDA;
+                g_nlaunch += s.graph_kernels;
+                mb[i].launched++;
+                any = true;
+            }
+        }
+        if (rc != HMFEM_OK) break;
+        if (ready < m) {  // the next one starts beside them
+            const int i = order[ready];
+            rc = batch_start(*ss[i], x ? x[i] : nullptr, mem, &mb[i].e0);
+            if (rc == HMFEM_OK) {
+                mb[i].runs = true;
+                ready++;
+                left++;
+            }
+            any = true;
+        } else if (done >= 0 && !any) {  // (the others' queues are full)
+            finish(done);
+            any = true;
+        }
+        if (any) {
+            polls = 0;
+            continue;
+        }
+        if (++polls % 256) continue;
+        sched_yield();
+        if (polls % 4096) continue;
+        for (int i = 0; i < m && rc == HMFEM_OK; i++) {  // (as in solve)
+            if (!mb[i].runs) continue;
+            const int at = *ss[i]->progress;
+            const cudaError_t e = cudaStreamQuery(ss[i]->st);
+            if (e == cudaSuccess && at >= 0 && *ss[i]->progress == at) finish(i);
+            if (e != cudaSuccess && e != cudaErrorNotReady) {
+                set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
+                rc = HMFEM_E_CUDA;
+            }
         }
     }
-    for (int i = 0; i < m; i++) {
-        if (ev[i]) cudaEventDestroy(ev[i]);
-        if (ev0[i]) cudaEventDestroy(ev0[i]);
-        if (cs[i]) cudaStreamDestroy(cs[i]);
+    for (int i = 0; i < m && rc != HMFEM_OK; i++) {  // nothing is left running
+        cudaStreamSynchronize(ss[i]->st);
+        if (mb[i].e0) cudaEventDestroy(mb[i].e0);
     }
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamSynchronize(ms);
-    cudaStreamDestroy(ms);
-    return rc != HMFEM_OK ? rc : worst;
+    for (int i = 0; i < m && rc == HMFEM_OK; i++) rc = status[i];
+    return rc;
 }
 
 // `iters` CG iterations from x = 0, launched without the graph, each

@@ -392,8 +392,8 @@ def iter_amg() -> int:
 
 
 def batch_solve(solvers, xs=None, allow_notconv=False):
-    """hmfem_batch_solve: set-up solvers solved together (one CUDA graph with
-    a branch per solver, replayed until all converged).  xs: per solver the
+    """hmfem_batch_solve: set-up solvers solved together (each on its own
+    stream, driven side by side by this thread).  xs: per solver the
     initial guess in / solution out (numpy arrays, or CUDA tensors), or None
     (zero guesses, nothing returned).  Returns the stats dicts."""
     L = lib()

@@ -118,7 +118,7 @@ typedef struct {
                           default 512); 0 =
                           the reference's diagonal solve on the coarsest
                           level (amg.h:1353-1364) */
-    int check_every;   /* host polls convergence every k iterations */
+    int check_every;   /* CG iterations queued beyond the last one done */
     int generic_setup; /* 1: coarsen an assembled level 0 with the generic
                           kernels and solve every level on SELL-32 (default
                           0: level 0 from its 7-point structure, levels 0-1
@@ -217,10 +217,9 @@ int hmfem_last_stats(hmfem_solver *s, hmfem_stats *st);
 int hmfem_time_kernel(hmfem_solver *s, int which, int level, int reps,
                       float *ms, double *bytes);
 
-/* Many set-up solvers solved together (batched uneven instances): one
- * CUDA graph holds one CG iteration of every solver, each on a branch of
- * its own, and is replayed until every solver has converged; a converged
- * solver's kernels return at once, so each stops at its own tolerance and
+/* Many set-up solvers solved together (batched uneven instances): each
+ * iterates on its own stream by its own captured iteration, side by side with
+ * the others and until its own tolerance, driven by the calling thread, and
  * gives the result it gives solved alone.  x[i]: solver i's initial guess
  * in, solution out (NULL array or entry: zero guess, nothing copied back);
  * st[i] (nullable) its stats.  Returns the first failing status. */
