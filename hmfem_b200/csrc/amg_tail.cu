@@ -18,7 +18,10 @@
 // steps, 2.1 -> 0.26 ms; 482 -> 1, five steps, 2.2 -> 0.40 ms.  Above 512 rows
 // the bit sets no longer fit, and one SM would soon take longer than the
 // general path's launches.
+#include <stdlib.h>
 #include <string.h>
+
+#include <algorithm>
 
 #include "hm.cuh"
 
@@ -43,9 +46,21 @@ struct TailLevel {
 };
 
 struct TailOut {
-    int levels;  // levels coarsened
+    int levels;    // levels coarsened
+    unsigned top;  // arena bytes in use after them
     TailLevel lv[kTailLevels];
 };
+
+// The arena's size; a smaller one when the environment sets
+// HMFEM_TEST_TAIL_ARENA (a test makes the levels run out of room and checks
+// that the general path goes on from there to the same hierarchy).
+size_t tail_arena_bytes()
+{
+    const char *e = getenv("HMFEM_TEST_TAIL_ARENA");
+    if (!e || !*e) return kTailArena;
+    const long long v = atoll(e);
+    return v < 0 ? 0 : std::min((size_t)v, kTailArena);
+}
 
 struct TailShared {
     double acc[kTailAcc];
@@ -125,12 +140,12 @@ __device__ void tail_ap(TailShared &S, int n, int nc, const int *rowptr, const i
 
 __global__ void __launch_bounds__(kTailThreads)
 k_tail(int n, const int *rowptr, const int *col, const double *val, int level, int max_levels,
-       int min_coarse, unsigned char *arena, unsigned cap, double *ap, TailOut *out)
+       int min_coarse, unsigned char *arena, unsigned top0, unsigned cap, double *ap, TailOut *out)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     TailShared &S = *(TailShared *)s_raw;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned top = 0;  // arena bytes in use (the same in every thread)
+    unsigned top = top0;  // arena bytes in use (the same in every thread)
     int done = 0;
     auto take = [&](size_t bytes) {
         const unsigned o = top;
@@ -308,7 +323,10 @@ k_tail(int n, const int *rowptr, const int *col, const double *val, int level, i
         __syncthreads();
         if (!more) break;
     }
-    if (tid == 0) out->levels = done;
+    if (tid == 0) {
+        out->levels = done;
+        out->top = top;
+    }
 }
 
 }  // namespace
@@ -324,6 +342,10 @@ int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, Tail
              cudaStream_t st, int *levels)
 {
     *levels = 0;
+    // A hierarchy may come here more than once (the arena was full, the general
+    // path made the next level): its earlier levels keep their place.
+    const size_t cap = tail_arena_bytes();
+    if (T.used >= cap) return HMFEM_OK;
     if (!T.mem) T.mem = (unsigned char *)dalloc(kTailArena);
     const Level &L0 = lv[l];
     double *ap = (double *)dalloc(sizeof(double) * (size_t)L0.A.n * L0.A.n);
@@ -335,8 +357,8 @@ int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, Tail
     HM_CUDA(cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(TailShared)));
     k_tail<<<1, kTailThreads, sizeof(TailShared), st>>>(
-        L0.A.n, L0.A.rowptr, L0.A.col, L0.A.val, l, max_levels, min_coarse, T.mem,
-        (unsigned)kTailArena, ap, out);
+        L0.A.n, L0.A.rowptr, L0.A.col, L0.A.val, l, max_levels, min_coarse, T.mem, T.used,
+        (unsigned)cap, ap, out);
     HM_LAUNCHED();
     static_assert(sizeof(TailOut) <= sizeof(int) * (PIN_WORDS - PIN_BLOCK), "pinned words");
     HM_CHECK(read_back(PIN_BLOCK, out, (int)(sizeof(TailOut) / sizeof(int)), st));
@@ -372,6 +394,7 @@ int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, Tail
         C.dinv = (double *)(T.mem + t.dinv);
         C.dinv32 = (float *)(T.mem + t.dinv32);
     }
+    T.used = h.top;
     *levels = h.levels;
     return HMFEM_OK;
 }

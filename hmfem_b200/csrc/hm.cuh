@@ -204,6 +204,7 @@ cudaStream_t side_stream();  // amg_setup.cu
 // general path has to go on)
 struct TailArena {
     unsigned char *mem = nullptr;  // kept by the solver; what setup made lies here
+    unsigned used = 0;             // bytes of it that the present hierarchy holds
 };
 bool tail_applies(const Level &L, int l);
 int amg_tail(std::vector<Level> &lv, int l, int max_levels, int min_coarse, TailArena &T,

@@ -289,6 +289,7 @@ static void free_hierarchy(Solver &s, bool keep_l0)
     s.dense_L = nullptr;
     s.direct_level = -1;
     s.small.first = -1;
+    s.tail.used = 0;
     s.nlevels = s.lv.size();
     s.setup_done = false;
     s.schur0_built = false;
