@@ -44,6 +44,10 @@ long long split_poll_limit()
 namespace {
 
 constexpr int kMisTile = 1024;
+// k_lfmis: a row gives up after max_polls polls, and not before the time that
+// many polls of an earlier tile take (measured ~1.2 us each): a poll of the
+// row's own tile is several times shorter, but it waits for the same chain.
+constexpr long long kPollCycles = 2400;
 
 // The greedy split in natural order (node_selection, amg.h:1-226 with
 // eps = 0): row v is C when every lower neighbour is F, F as soon as one is
@@ -94,6 +98,7 @@ k_lfmis(const int *__restrict__ rowptr, const int *__restrict__ col, int n,
         if (t == 0) (u >= base ? near : far) |= 1ull << p;
     }
     long long polls = 0;
+    const long long t0 = clock64();
     int pn = -1, pf = -1;
     for (unsigned it = 0; !isF; it++) {
         if (near && (it % 2 == 0 || !far)) {
@@ -139,7 +144,11 @@ k_lfmis(const int *__restrict__ rowptr, const int *__restrict__ col, int n,
             if (polls > 32) __nanosleep(64);
         }
         // (the error word lies in global memory: looked at now and then)
-        if (++polls > max_polls || (polls % 256 == 0 && *verr)) { atomicExch(err, 1); return; }
+        if ((++polls > max_polls && clock64() - t0 > max_polls * kPollCycles) ||
+            (polls % 256 == 0 && *verr)) {
+            atomicExch(err, 1);
+            return;
+        }
     }
     const signed char d = isF ? 2 : 1;
     ss[threadIdx.x] = d;
