@@ -666,15 +666,24 @@ static int capture_iteration(Solver &s)
         return rc;
     }
     HM_CUDA(e);
-    s.graph = g;
     if (s.gexec) {
         cudaGraphExecUpdateResultInfo info;
-        if (cudaGraphExecUpdate(s.gexec, g, &info) == cudaSuccess) return HMFEM_OK;
+        if (cudaGraphExecUpdate(s.gexec, g, &info) == cudaSuccess) {
+            s.graph = g;
+            return HMFEM_OK;
+        }
         cudaGetLastError();  // another graph: instantiate it
         cudaGraphExecDestroy(s.gexec);
         s.gexec = nullptr;
     }
-    HM_CUDA(cudaGraphInstantiate(&s.gexec, g, 0));
+    e = cudaGraphInstantiate(&s.gexec, g, 0);
+    if (e != cudaSuccess) {  // (s.graph stays null: the next solve captures again)
+        s.gexec = nullptr;
+        cudaGraphDestroy(g);
+        cudaGetLastError();  // (reported here; the next launch starts clean)
+    }
+    HM_CUDA(e);
+    s.graph = g;
     return HMFEM_OK;
 }
 
