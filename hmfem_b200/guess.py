@@ -136,6 +136,8 @@ def relu_grad_raw(gout, out):
     """(g, gb): g = gout * (out > 0) (out None: g is gout) and its sums over
     the cells (FP32); gout, out (c/8, n, 8) bf16."""
     gout = gout.contiguous()
+    if gout.data_ptr() % 16:  # a view into a larger buffer: the kernels want 16 bytes
+        gout = gout.clone()
     slabs, n, _ = gout.shape
     g = gout if out is None else torch.empty_like(gout)
     gb = torch.empty(8 * slabs, dtype=torch.float32, device=gout.device)
