@@ -784,7 +784,14 @@ k_conv3d(const __nv_bfloat16 *__restrict__ in, const __grid_constant__ CUtensorM
 // part's D in tensor memory over all its cells and adds it into dw at the
 // end.  Roles: warp 4 loads (a lane per group), warp 5 issues, warps 0-3
 // read D.
+//
+// The zeros outside the grid are multiplied like cells, and zero times a
+// non-finite cell is NaN: entries of D that come out NaN where the CTA meets
+// the grid's edge are summed again over its pairs of cells that both lie in
+// the grid (wgrad_nan_entries), so only those pairs count whatever the cells
+// hold.
 struct WgPlan {
+    int nx, ny, nz;
     int flip;              // 0: M = x, N = dy; 1: M = dy, N = x
     int ms, gm, gmax;      // M side: slabs, groups (3 ms), groups per stage
     int mb;                // groups per copy: divides ms and 16
@@ -813,12 +820,78 @@ __host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n)
     return idesc_bf16(m, n) | (1u << 15) | (1u << 16);
 }
 
+// Whether any step of CTA idx multiplies, in the entries of shift (i, j, k), a
+// cell of the grid with a place outside it.
+template <int BY>
+__device__ __noinline__ bool wgrad_meets_edge(const WgPlan &p, int idx, int i, int j, int k)
+{
+    for (long it = idx; it < (long)p.nxc * p.nyb * p.nzc; it += p.per) {
+        const int xc = (int)(it % p.nxc), yb = (int)((it / p.nxc) % p.nyb),
+                  zc = (int)(it / ((long)p.nxc * p.nyb));
+        const bool xe = xc == p.nxc - 1, ye = yb == p.nyb - 1;
+        if (i == 0 ? xc == 0 || (xe && p.nx % 32) : i == 2 && xe) return true;
+        if (j == 0 ? yb == 0 || (ye && p.ny % BY) : j == 2 && ye) return true;
+        if (k == 0 ? zc == 0 : k == 2 && zc == p.nzc - 1) return true;
+    }
+    return false;
+}
+
+// Eight entries of CTA idx's D, sum_p M[p + (i-1)][cm] N[p + (j-1, k-1)][8 slab
+// + 0..7] over its steps without the pairs of which a cell lies outside the
+// grid: a warp, a lane per cell of a row.  Left as soon as all eight are NaN.
+struct Entries {
+    float v[8];
+};
+template <int BY>
+__device__ __noinline__ Entries wgrad_nan_entries(const __nv_bfloat16 *__restrict__ m,
+                                                  const __nv_bfloat16 *__restrict__ nn,
+                                                  const WgPlan &p, int idx, int cm, int slab,
+                                                  int i, int j, int k)
+{
+    const int lane = threadIdx.x & 31;
+    const long nx = p.nx, nxy = nx * p.ny, cells = nxy * p.nz;
+    double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    bool nan = false;
+    for (long it = idx; it < (long)p.nxc * p.nyb * p.nzc && !nan; it += p.per) {
+        const int xc = (int)(it % p.nxc), yb = (int)((it / p.nxc) % p.nyb),
+                  zc = (int)(it / ((long)p.nxc * p.nyb));
+        const int x = 32 * xc + lane;
+        const bool on = x >= (i == 0) && x < p.nx - (i == 2);
+        const int y0 = max(BY * yb, j == 0), y1 = min(BY * yb + BY, p.ny - (j == 2));
+        const int z0 = max(p.zl * zc, k == 0), z1 = min(p.zl * zc + p.zl, p.nz - (k == 2));
+        for (int z = z0; z < z1 && !nan; z++) {
+#pragma unroll
+            for (int r = 0; r < BY; r++) {
+                const int y = BY * yb + r;
+                if (!on || y < y0 || y >= y1) continue;
+                const long c = x + y * nx + z * nxy;
+                const double a = (double)__bfloat162float(
+                    m[((cm / 8) * cells + c + i - 1) * 8 + cm % 8]);
+                const uint4 q = ((const uint4 *)nn)[slab * cells + c + (j - 1) * nx +
+                                                    (k - 1) * nxy];
+                const __nv_bfloat16 *e = (const __nv_bfloat16 *)&q;
+#pragma unroll
+                for (int w = 0; w < 8; w++) t[w] += a * (double)__bfloat162float(e[w]);
+            }
+            nan = true;
+#pragma unroll
+            for (int w = 0; w < 8; w++) nan = __any_sync(0xffffffffu, t[w] != t[w]) && nan;
+        }
+    }
+    Entries f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) f.v[w] = (float)__shfl_sync(0xffffffffu, warp_sum(t[w]), 0);
+    return f;
+}
+
 template <int NS, int BY>
 __global__ void __launch_bounds__(kConvThreads, 1)
 k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_n,
-        float *__restrict__ dw, int nz, const WgPlan p, int *err)
+        const __nv_bfloat16 *__restrict__ gm, const __nv_bfloat16 *__restrict__ gn,
+        float *__restrict__ dw, const __grid_constant__ WgPlan p, int *err)
 {
     using C = WgCfg<NS, BY>;
+    const int nz = p.nz;
     constexpr int SP = C::SP, GN = C::GN, RM = C::RM, RN = C::RN;
     extern __shared__ __align__(128) unsigned char smem[];
     const int mstage = p.gmax * SP;
@@ -977,11 +1050,27 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
         for (int c = 0; c < C::COLS; c += 16) {
             float f[16];
             tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, f);
-            if (!v) continue;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const int q = c / 8 + h, k = q / GN, j = (q / NS) % 3;
-                const int cn = 8 * (s0 + q % NS);
+                const int q = c / 8 + h, k = q / GN, j = (q / NS) % 3, sn = s0 + q % NS;
+                const int cn = 8 * sn;
+                const float t = ((f[8 * h] + f[8 * h + 1]) + (f[8 * h + 2] + f[8 * h + 3])) +
+                                ((f[8 * h + 4] + f[8 * h + 5]) + (f[8 * h + 6] + f[8 * h + 7]));
+                if (__any_sync(0xffffffffu, t != t)) {
+                    // a row at a time, by the warp
+                    unsigned rows = __ballot_sync(
+                        0xffffffffu, v && t != t && wgrad_meets_edge<BY>(p, idx, i, j, k));
+                    for (; rows; rows &= rows - 1) {
+                        const int r = __ffs(rows) - 1;
+                        const Entries n = wgrad_nan_entries<BY>(
+                            gm, gn, p, idx, __shfl_sync(0xffffffffu, cm, r), sn,
+                            __shfl_sync(0xffffffffu, i, r), j, k);
+#pragma unroll
+                        for (int e = 0; e < 8; e++)
+                            if (lane == r) f[8 * h + e] = n.v[e];
+                    }
+                }
+                if (!v) continue;
                 if (!p.flip) {
                     // X at p + (i-1), dY at p + (j-1, k-1): tap (i-1, 1-j, 1-k)
                     const int tap = 9 * (2 - k) + 3 * (2 - j) + i;
@@ -1230,6 +1319,9 @@ int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, i
                      int nz, WgPlan p, int nsm, int *err, cudaStream_t st)
 {
     using C = WgCfg<NS, BY>;
+    p.nx = nx;
+    p.ny = ny;
+    p.nz = nz;
     p.ms = cm / 8;
     p.gm = 3 * p.ms;
     p.gmax = p.gm < 16 ? p.gm : 16;
@@ -1277,7 +1369,8 @@ int launch_wgrad_cfg(const void *m, const void *nn, int cm, int cn, float *dw, i
     static_assert(16 * C::SP <= C::RN * C::GN * C::SP, "operand overrun");
     auto k = k_wgrad<NS, BY>;
     HM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    k<<<(unsigned)(per * p.parts), kConvThreads, bytes, st>>>(tm[0], tm[1], dw, nz, p, err);
+    k<<<(unsigned)(per * p.parts), kConvThreads, bytes, st>>>(
+        tm[0], tm[1], (const __nv_bfloat16 *)m, (const __nv_bfloat16 *)nn, dw, p, err);
     HM_LAUNCHED();
     return HMFEM_OK;
 }

@@ -39,7 +39,9 @@ int hmfem_conv3d_plan(int nx, int ny, int nz, int cin, int cout, int nsm, int sm
                       int *plan);
 
 /* dw[27][cout][cin] += sum over cells of dy[cell][co] x[cell + tap][ci] (the
- * weight gradient), FP32, on the tensor cores. */
+ * weight gradient), FP32, on the tensor cores.  The sum is over the cells
+ * whose cell + tap lies in the grid: beyond it nothing is added, not even
+ * where the other factor is infinite or NaN. */
 int hmfem_conv3d_wgrad(const void *x, const void *dy, float *dw, int nx, int ny, int nz,
                        int cin, int cout, int *err, void *stream);
 
