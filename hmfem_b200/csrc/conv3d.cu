@@ -1432,6 +1432,16 @@ int hmfem_conv3d_plan(int nx, int ny, int nz, int cin, int cout, int nsm, int sm
     return p.ns >= 1 ? HMFEM_OK : HMFEM_E_ARG;
 }
 
+int hmfem_conv3d_plan_zg(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_max, int *zg)
+{
+    if (!zg || nx < 1 || ny < 1 || nz < 1 || cin < 16 || cin % 16 || cout < 16 ||
+        cout % 16 || cout > 256 || nsm < 1 || smem_max < 1024)
+        return HMFEM_E_ARG;
+    const hm::ConvPlan p = hm::plan_conv(nx, ny, nz, cin, cout, nsm, smem_max);
+    *zg = p.zg;
+    return p.ns >= 1 ? HMFEM_OK : HMFEM_E_ARG;
+}
+
 int hmfem_conv3d_wgrad(const void *x, const void *dy, float *dw, int nx, int ny, int nz,
                        int cin, int cout, int *err, void *stream)
 {

@@ -41,6 +41,7 @@ def _lib():
         L.hmfem_conv3d_fwd.argtypes = [vp, vp, vp, vp, i, i, i, i, i, i, vp, vp]
         L.hmfem_conv3d_wgrad.argtypes = [vp, vp, vp, i, i, i, i, i, vp, vp]
         L.hmfem_conv3d_plan.argtypes = [i, i, i, i, i, i, i, vp]
+        L.hmfem_conv3d_plan_zg.argtypes = [i, i, i, i, i, i, i, vp]
         L.hmfem_guess_features.argtypes = [vp, vp, i, i, i, vp, vp]
         L.hmfem_guess_pool2.argtypes = [vp, i, i, i, i, vp, vp]
         L.hmfem_guess_up2_cat.argtypes = [vp, i, vp, i, i, i, i, vp, vp]
@@ -63,7 +64,10 @@ def conv_plan(dims, cin, cout, nsm=148, smem_max=232448):
                                   C.addressof(out))
     if rc != 0:
         raise gpu.HmfemError(rc, gpu.last_error())
-    return dict(zip(PLAN_FIELDS, list(out)))
+    zg = C.c_int()
+    _lib().hmfem_conv3d_plan_zg(dims[0], dims[1], dims[2], cin, cout, nsm, smem_max,
+                                C.addressof(zg))
+    return dict(zip(PLAN_FIELDS, list(out)), zg=zg.value)
 
 
 _ERR = {}

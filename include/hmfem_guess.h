@@ -37,6 +37,10 @@ int hmfem_conv3d_fwd(const void *in, const void *w, const float *bias, void *out
  * the three x taps of each (dy, dz) share one MMA (N = 3 Cout). */
 int hmfem_conv3d_plan(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_max,
                       int *plan);
+/* *zg = 1 when that launch adds an input plane into up to three output planes
+ * by one MMA (the z taps of each (dx, dy): N = Cout to 3 Cout). */
+int hmfem_conv3d_plan_zg(int nx, int ny, int nz, int cin, int cout, int nsm, int smem_max,
+                         int *zg);
 
 /* dw[27][cout][cin] += sum over cells of dy[cell][co] x[cell + tap][ci] (the
  * weight gradient), FP32, on the tensor cores.  The sum is over the cells
