@@ -1042,7 +1042,11 @@ static int cycle_t(Solver &s, int l, cudaStream_t st, bool dot, bool seeded)
         return HMFEM_OK;
     }
     // from here down in one launch, where the levels fit
-    if (l == s.small.first && (s.small.kind == 0) == std::is_same<T, double>::value && seeded) {
+    if (l == s.small.first && (s.small.kind == 0) == std::is_same<T, double>::value) {
+        if (!seeded) {  // (a cycle that starts here)
+            launch_pdl(k_seed<T>, nb(n), 256, st, n, f, seed_of<T>(s, l));
+            HM_LAUNCHED();
+        }
         const ChebCoef cc = cheb_coef(s.opt.cheb_degree);
         return small_cycle(s, cc.c1, cc.c2, cc.ith, ctl, st);
     }
@@ -1440,7 +1444,10 @@ __global__ void k_fill_one(double *x, int n)
 //  11 Chebyshev step FP64 (coarse level, SELL)  nnz*(8+4) + n*8*7
 //     (d gathered, D^-1, r and u read and written, d' written)
 // and 12: one whole V-cycle from level l in the solver's precision (bytes
-// reported 0); the difference between levels l and l+1 is level l's share.
+// reported 0); the difference between levels l and l+1 is level l's share down
+// to the first level of the one-launch form (small_cycle.cu), whose time is
+// that launch: levels below it have no share of their own, and from them the
+// cycle runs the level kernels, which a solve does not.
 int time_kernel(Solver &s, int which, int l, int reps, float *ms, double *bytes)
 {
     // (levels below the coarse solve have no solve-phase forms until now)
