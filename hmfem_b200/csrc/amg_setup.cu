@@ -74,7 +74,11 @@ k_lfmis(const int *__restrict__ rowptr, const int *__restrict__ col, int n,
 {
     __shared__ int s_tile;
     __shared__ signed char s_sel[kMisTile];
-    if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
+    __shared__ long long s_t0;
+    if (threadIdx.x == 0) {
+        s_tile = (int)atomicAdd(ticket, 1u);
+        s_t0 = clock64();
+    }
     s_sel[threadIdx.x] = 0;
     __syncthreads();
     const long base = (long)s_tile * kMisTile;
@@ -98,7 +102,6 @@ k_lfmis(const int *__restrict__ rowptr, const int *__restrict__ col, int n,
         if (t == 0) (u >= base ? near : far) |= 1ull << p;
     }
     long long polls = 0;
-    const long long t0 = clock64();
     int pn = -1, pf = -1;
     for (unsigned it = 0; !isF; it++) {
         if (near && (it % 2 == 0 || !far)) {
@@ -144,7 +147,7 @@ k_lfmis(const int *__restrict__ rowptr, const int *__restrict__ col, int n,
             if (polls > 32) __nanosleep(64);
         }
         // (the error word lies in global memory: looked at now and then)
-        if ((++polls > max_polls && clock64() - t0 > max_polls * kPollCycles) ||
+        if ((++polls > max_polls && clock64() - s_t0 > max_polls * kPollCycles) ||
             (polls % 256 == 0 && *verr)) {
             atomicExch(err, 1);
             return;
