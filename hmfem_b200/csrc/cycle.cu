@@ -14,6 +14,18 @@ namespace hm {
 
 thread_local std::vector<KRec> *t_kprof = nullptr;
 thread_local int t_pdl_blocks = 296;
+
+int pdl_blocks_for(long n0)
+{
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 148;
+    }();
+    return sms * (ceil_div(n0, 256) <= 5 * sms ? 5 : 2);
+}
+
 thread_local int t_klevel = -1;
 
 int g_pdl = [] {

@@ -73,13 +73,22 @@ extern int g_pdl;  // 0: plain stream order (HMFEM_PDL=0)
 // Only launches of a limited size are scheduled early: a small kernel gains
 // its launch latency, but the blocks of a large one that wait on the SMs take
 // room from the kernel that still runs.  One CG iteration (us) with every
-// launch early / none / up to 296 blocks: 256^3 reduced precision 1304 / 1237
-// / 1228, 256^3 FP64 2375 / 2302 / 2296, 128^3 reduced 297 / 289 / 282, 32^3
-// FP64 67 / 77 / 67.  Where level 0 itself is one pass of short kernels (up to
-// ~180000 rows) the limit lies above it: the coupled run at 210x42x20 takes
-// 199 ms with 296, 191 with 700, and 128^3 15.1 against 14.9 with 700.
+// launch early / none / up to two blocks per SM: 256^3 reduced precision 1304 /
+// 1237 / 1228, 256^3 FP64 2375 / 2302 / 2296, 128^3 reduced 297 / 289 / 282,
+// 32^3 FP64 67 / 77 / 67.
+// Where level 0 itself has no more than five blocks per SM (189440 rows) every
+// launch is early.  Two blocks per SM / 704 blocks (all of them early up to
+// 180224 rows), FP64 and reduced precision:
+//     rows      FP64          reduced       rows      FP64          reduced
+//     64000   83.5 /  84.1  72.4 /  71.2   216000  117.9 / 116.3  103.6 / 103.2
+//     97336   97.8 /  96.2  80.3 /  77.2   262144  124.4 / 128.1  109.7 / 112.8
+//    130000  104.4 / 102.1  84.0 /  80.5   268800  126.1 / 130.1  112.2 / 114.9
+//    176400  107.7 / 104.9  97.2 /  94.0   983040  268.6 / 273.5  185.7 / 188.5
+// (216000 rows with all early: 117.3 and 102.1; 268800: 130.0 and 115.2.)  Past
+// five, a single early pass of 500 to 700 blocks loses 2-5 % where a level has
+// one, and three or four blocks per SM are as good as two within 2 %.
 extern thread_local int t_pdl_blocks;
-inline int pdl_blocks_for(long n0) { return n0 <= 180000 ? 704 : 296; }
+int pdl_blocks_for(long n0);
 
 // Per-launch timing of the solve phase (hmfem_profile_iteration): while
 // t_kprof is set on a host thread, launch_pdl brackets each of its launches
