@@ -1240,8 +1240,10 @@ int hmfem_set_matrix(hmfem_solver *h, int n, long nnz, const int *cnt,
         HM_ALLOC(cl, int, nnz);
         HM_ALLOC(vl, double, nnz);
         HM_CHECK(hm::upload(rp, cnt, n, mem, st));
-        long tot = 0;
-        HM_CHECK(hm::rowptr_from_counts(rp, n, st, &tot));
+        long tot = -1;
+        // (counts that are no matrix are refused below)
+        const int rc = hm::rowptr_from_counts(rp, n, st, &tot);
+        if (rc != HMFEM_E_CAPACITY) HM_CHECK(rc);
         bool same = false;
         if (tot == nnz) {
             HM_CHECK(hm::upload(cl, col, nnz, mem, st));
@@ -1269,11 +1271,12 @@ int hmfem_set_matrix(hmfem_solver *h, int n, long nnz, const int *cnt,
     HM_CHECK(hm::launch_validate_counts(L.A.rowptr, n, s.dwork + 9, st));
     HM_CUDA(cudaMemcpyAsync(&bad, s.dwork + 9, sizeof(int), cudaMemcpyDeviceToHost, st));
     long tot = 0;
-    HM_CHECK(hm::rowptr_from_counts(L.A.rowptr, n, st, &tot));  // synchronises
-    if (bad) {
+    const int rc = hm::rowptr_from_counts(L.A.rowptr, n, st, &tot);  // synchronises
+    if (bad) {  // (their sum may look like a wrapped one)
         hm::set_last_error("negative row count", __FILE__, __LINE__);
         return HMFEM_E_ARG;
     }
+    HM_CHECK(rc);
     if (tot != nnz) {
         hm::set_last_error("row counts do not add up to hdr[1]", __FILE__, __LINE__);
         return HMFEM_E_ARG;
