@@ -900,9 +900,13 @@ int batch_solve(Solver *const *ss, int m, double *const *x, int mem, hmfem_stats
         if (polls % 4096) continue;
         for (int i = 0; i < m && rc == HMFEM_OK; i++) {  // (as in solve)
             if (!mb[i].runs) continue;
+            // (a member that got on since the pass above, while this thread
+            // was away, is only waiting for its next launch)
+            const int ahead = ss[i]->opt.check_every > 0 ? ss[i]->opt.check_every : 4;
             const int at = *ss[i]->progress;
+            if (at < 0 || mb[i].launched - at < ahead) continue;
             const cudaError_t e = cudaStreamQuery(ss[i]->st);
-            if (e == cudaSuccess && at >= 0 && *ss[i]->progress == at) finish(i);
+            if (e == cudaSuccess && *ss[i]->progress == at) finish(i);
             if (e != cudaSuccess && e != cudaErrorNotReady) {
                 set_last_error(cudaGetErrorString(e), __FILE__, __LINE__);
                 rc = HMFEM_E_CUDA;
