@@ -733,7 +733,7 @@ int solve(Solver &s, const double *b, double *x, int mem, hmfem_stats *out)
     int launched = 0;
     for (unsigned polls = 0;;) {
         const int at = *s.progress;
-        if (at < 0 || launched > s.opt.max_iter + 2 * ahead) break;
+        if (at < 0 || launched > s.opt.max_iter + 2l * ahead) break;
         if (launched - at < ahead) {
             HM_CUDA(cudaGraphLaunch(s.gexec, st));
             g_nlaunch += s.graph_kernels;
@@ -868,7 +868,7 @@ int batch_solve(Solver *const *ss, int m, double *const *x, int mem, hmfem_stats
             Solver &s = *ss[i];
             const int ahead = s.opt.check_every > 0 ? s.opt.check_every : 4;
             const int at = *s.progress;
-            if (at < 0 || mb[i].launched > s.opt.max_iter + 2 * ahead) {
+            if (at < 0 || mb[i].launched > s.opt.max_iter + 2l * ahead) {
                 done = i;
             } else if (mb[i].launched - at < ahead) {
                 if (cudaGraphLaunch(s.gexec, s.st) != cudaSuccess) rc = HMFEM_E_CUDA;
