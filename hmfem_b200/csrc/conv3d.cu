@@ -1049,6 +1049,7 @@ k_wgrad(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtens
 #pragma unroll 1
         for (int c = 0; c < C::COLS; c += 16) {
             float f[16];
+            __syncwarp();  // (rows beyond the tensor's skip the stores; the read is the warp's)
             tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, f);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
