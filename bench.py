@@ -1120,6 +1120,12 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", 0))
     if rank != 0:
         return
+    from oracle import oracle
+    if not os.path.exists(oracle.REF_SO):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "oracle/_ref/libhmfem_ref.so is not there (it is compiled from the "
+                          "reference's own sources)"}), flush=True)
+        return
     import multiprocessing as mp
     size = args.size
     per_gb = 14.0 * (size / 256.0) ** 3 + 0.5
